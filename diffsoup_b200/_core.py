@@ -65,6 +65,7 @@ _sig("ds_backward_multires_triangle_alpha", _i32, _i32, _vp, _i32, _i32, _i32, _
 _sig("ds_multires_triangle_color", _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_backward_multires_triangle_color", _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_accumulate_to_level_forward", _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
+_sig("ds_accumulate_to_level_backward_set", _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_accumulate_to_level_backward", _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_make_view_table", _i32, _i32, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(ViewDesc),
      C.POINTER(C.c_int64))
@@ -238,6 +239,14 @@ def accumulate_to_level_backward(min_level: int, max_level: int, target_level: i
     T, S, Cd = grad_feat_all.shape
     check(_lib.ds_accumulate_to_level_backward(T, min_level, max_level, target_level, S, grad_feat_max.shape[1], Cd,
                                                ptr(grad_feat_all), ptr(grad_feat_max), stream()))
+
+
+def accumulate_to_level_backward_set(min_level: int, max_level: int, target_level: int, grad_feat_all,
+                                     grad_feat_max) -> None:
+    """accumulate_to_level_backward into an uninitialised gradient buffer (overwritten)."""
+    T, S, Cd = grad_feat_all.shape
+    check(_lib.ds_accumulate_to_level_backward_set(T, min_level, max_level, target_level, S, grad_feat_max.shape[1],
+                                                   Cd, ptr(grad_feat_all), ptr(grad_feat_max), stream()))
 
 
 def split_triangle_soup(verts, faces, numSplits: int, tau: float):

@@ -189,8 +189,8 @@ class _AccumulateToLevelFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         lo, hi, tl = ctx.levels
-        grad_feat = torch.zeros(ctx.feat_shape, dtype=torch.float32, device=grad_out.device)
-        _core.accumulate_to_level_backward(lo, hi, tl, grad_feat, grad_out.contiguous())
+        grad_feat = torch.empty(ctx.feat_shape, dtype=torch.float32, device=grad_out.device)
+        _core.accumulate_to_level_backward_set(lo, hi, tl, grad_feat, grad_out.contiguous())
         return None, None, None, grad_feat
 
 

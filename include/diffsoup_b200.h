@@ -146,6 +146,11 @@ int ds_accumulate_to_level_forward(int T, int min_level, int max_level, int targ
 int ds_accumulate_to_level_backward(int T, int min_level, int max_level, int target_level, int S, int S_target,
                                     int C, float* grad_features, const float* grad_out, ds_stream_t stream);
 
+/* The same gradient with grad_features [T,S,C] overwritten (no zeroed buffer
+ * needed), for callers that want it alone. */
+int ds_accumulate_to_level_backward_set(int T, int min_level, int max_level, int target_level, int S, int S_target,
+                                        int C, float* grad_features, const float* grad_out, ds_stream_t stream);
+
 /* ===================================================================== */
 /*  B200 path: screen-tile binning, tiled rasterizer, tiled aux gradient  */
 /* ===================================================================== */
