@@ -27,7 +27,7 @@ constexpr int kWarpsPerCta = 8;
 constexpr int kBlocksPerTile = 8;  // 32-pixel blocks of a 16x16 tile, one warp each
 static_assert(DS_TILE == 16, "the block decode of block_geometry assumes 16x16 tiles");
 constexpr int kSortMax = 512;      // longest tile list sorted by depth
-constexpr int kSortWarps = 8;      // warps (tiles) per CTA of the sort pass
+constexpr int kSortWarps = 4;      // warps (tiles) per CTA of the sort pass
 
 // One entry of a tile's list: the (view, triangle) record's pixel rect and
 // near depth bound, and the record index -- what the rasterizer's staging
@@ -131,16 +131,33 @@ __device__ __forceinline__ void warp_items(int n, F&& f) {
     }
 }
 
+// Triangles per warp of the two binning passes.  A warp's time is a chain of
+// items / 32 dependent rounds, so when 32 triangles a warp would leave most of
+// the chip without a warp, a warp takes 8 (its first lanes own one each, all
+// lanes work on their tiles).  At 15,000 pairs (one 1200x1200 view) 8 a warp
+// took the two passes from 59 to 22 us (with the fill pass below); at 120,000
+// (8 views of 800x800) 32 a warp took 43 us and 8 a warp 57 us.
+constexpr int64_t kBinNarrow = 60000;  // (view, triangle) pairs up to which a warp takes 8
+
+// Record index of the calling lane, or n for a lane without one.
+template <int TPW>
+__device__ __forceinline__ int64_t bin_record(int64_t n) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * TPW + lane;
+    return lane < TPW && i < n ? i : n;
+}
+
 // Pass 1: boxes, vertices, depth bounds, edge records and per-tile counts.
-// The (triangle, tile) pairs of a warp's 32 triangles are tested 32 at a
+// The (triangle, tile) pairs of a warp's triangles are tested 32 at a
 // time (warp_items), so lanes do not wait on the lane with the largest rect.
+template <int TPW>
 __global__ void __launch_bounds__(kThreads) bin_setup_kernel(int B, const ds_view_desc* __restrict__ views, int V,
                                                              const float* __restrict__ pos, int T,
                                                              const int* __restrict__ tri, TriBox* __restrict__ boxes,
                                                              TriVerts* __restrict__ verts, TriNdc* __restrict__ ndc,
                                                              TriEdges* __restrict__ edges, int* __restrict__ counts) {
     __shared__ unsigned long long s_mask[kThreads];
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = bin_record<TPW>((int64_t)B * T);
     const bool live = i < (int64_t)B * T;
     const int b = live ? (int)(i / T) : 0, t = live ? (int)(i % T) : 0;
     const ds_view_desc vd = views[b];
@@ -218,9 +235,37 @@ __global__ void __launch_bounds__(kThreads) bin_setup_kernel(int B, const ds_vie
     edges[i] = te;
 }
 
+// Bit position of the k-th set bit of m (k < popcount), by halving the word.
+__device__ __forceinline__ int select_bit(uint64_t m, int k) {
+    const int nlo = __popc((uint32_t)m);
+    const bool up = k >= nlo;
+    uint32_t w = up ? (uint32_t)(m >> 32) : (uint32_t)m;
+    k -= up ? nlo : 0;
+    int at = up ? 32 : 0;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+        const int c = __popc(w & ((1u << h) - 1u));
+        const bool hi = k >= c;
+        k -= hi ? c : 0;
+        at += hi ? h : 0;
+        w = hi ? w >> h : w;
+    }
+    return at;
+}
+
 // Pass 2: scatter record indices into the per-tile lists: the tiles of the
-// count pass's masks, distributed over the warp (warp_items), and for rects
-// of more than 64 tiles the test itself, per triangle.
+// count pass's masks, distributed over the warp, and for rects of more than
+// 64 tiles the test itself, one triangle at a time with its tiles over the
+// lanes.  An entry is a chain of two dependent global round trips (the list's
+// start and the cursor's atomic, then the store), so each lane keeps kFillItems
+// of them in flight.  Together with the bit selection
+// and the shared large rects: 200,000 triangles in 3 views of 1920x1080
+// (5,237 rects of more than 64 tiles) 369 -> 45 us, 360,000 pairs in 6 uneven views
+// 101 -> 20 us, one 1200x1200 view 37 -> 9.5 us; 120,000 pairs without a
+// large rect stay at 13-15 us.
+constexpr int kFillItems = 4;
+
+template <int TPW>
 __global__ void __launch_bounds__(kThreads) bin_fill_kernel(int B, const ds_view_desc* __restrict__ views, int T,
                                                             const TriBox* __restrict__ boxes,
                                                             const TriVerts* __restrict__ verts,
@@ -228,11 +273,11 @@ __global__ void __launch_bounds__(kThreads) bin_fill_kernel(int B, const ds_view
                                                             const int64_t* __restrict__ offsets,
                                                             int* __restrict__ cursor, ListEntry* __restrict__ list,
                                                             int64_t capacity, int* __restrict__ status) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int64_t i = bin_record<TPW>((int64_t)B * T);
     const bool live = i < (int64_t)B * T;
     const int b = live ? (int)(i / T) : 0;
-    const ds_view_desc vd = views[b];
-    int tx0 = 0, tx1 = -1, ty0 = 0, ty1 = -1;
+    int ntx = 0, nty = 0, org = 0, pitch = 0;  // the rect in tiles; the tile of its corner, tiles per row of its view
     uint64_t m = 0;
     ListEntry le;
     le.y0 = le.y1 = le.x0 = le.x1 = 0;
@@ -242,44 +287,83 @@ __global__ void __launch_bounds__(kThreads) bin_fill_kernel(int B, const ds_view
         const TriBox rc = boxes[i];
         le.y0 = rc.y0; le.y1 = rc.y1; le.x0 = rc.x0; le.x1 = rc.x1;
         le.zlo = rc.zlo;
+        int tx0, tx1, ty0, ty1;
         if (box_tiles(rc, tx0, tx1, ty0, ty1)) {
             const float4 nb = ndc[i].b;
             m = (uint64_t)__float_as_uint(nb.z) | ((uint64_t)__float_as_uint(nb.w) << 32);
-        } else {
-            tx1 = tx0 - 1;
-            ty1 = ty0 - 1;
+            ntx = tx1 - tx0 + 1;
+            nty = ty1 - ty0 + 1;
+            pitch = views[b].tiles_x;
+            org = views[b].tile_base + ty0 * pitch + tx0;
         }
     }
-    const int ntx = tx1 - tx0 + 1, nty = ty1 - ty0 + 1;
-    const int ntiles = ntx > 0 && nty > 0 ? ntx * nty : 0;
-    const bool small = ntiles <= 64;
+    const bool small = ntx * nty <= 64;
     bool over = false;
-    const uint32_t mlo = (uint32_t)m, mhi = (uint32_t)(m >> 32);
     const int4 lw = *reinterpret_cast<const int4*>(&le);
-    warp_items(small ? __popcll(m) : 0, [&](bool valid, int owner, int k) {
-        const uint32_t olo = __shfl_sync(0xffffffffu, mlo, owner), ohi = __shfl_sync(0xffffffffu, mhi, owner);
-        const int4 ole = make_int4(__shfl_sync(0xffffffffu, lw.x, owner), __shfl_sync(0xffffffffu, lw.y, owner),
-                                   __shfl_sync(0xffffffffu, lw.z, owner), __shfl_sync(0xffffffffu, lw.w, owner));
-        const int otx0 = __shfl_sync(0xffffffffu, tx0, owner), oty0 = __shfl_sync(0xffffffffu, ty0, owner);
-        const int ontx = __shfl_sync(0xffffffffu, ntx, owner), ob = __shfl_sync(0xffffffffu, b, owner);
-        if (!valid) return;
-        // the k-th tile of the owner's mask
-        const int nlo = __popc(olo);
-        const int bit = k < nlo ? (int)__fns(olo, 0, k + 1) : 32 + (int)__fns(ohi, 0, k - nlo + 1);
-        const ds_view_desc ovd = views[ob];
-        const int tile = ovd.tile_base + (oty0 + bit / ontx) * ovd.tiles_x + otx0 + bit % ontx;
-        const int64_t at = offsets[tile] + atomicAdd(cursor + tile, 1);
-        if (at < capacity) *reinterpret_cast<int4*>(list + at) = ole;
-        else over = true;
-    });
-    if (live && !small) {  // large rects: the test itself
-        for (int ty = ty0; ty <= ty1; ++ty)
-            for (int tx = tx0; tx <= tx1; ++tx) {
-                if (!tile_may_cover(verts[i], vd, tx, ty)) continue;
-                const int tile = vd.tile_base + ty * vd.tiles_x + tx;
-                const int64_t at = offsets[tile] + atomicAdd(cursor + tile, 1);
-                if (at < capacity) list[at] = le; else over = true;
+    const uint32_t mlo = (uint32_t)m, mhi = (uint32_t)(m >> 32);
+    int excl = small ? __popcll(m) : 0;
+    const int mine = excl;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, excl, o);
+        if (lane >= o) excl += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, excl, 31);
+    excl -= mine;  // first item of this lane
+    for (int base = 0; base < total; base += 32 * kFillItems) {
+        int tile[kFillItems];
+        int4 ent[kFillItems];
+#pragma unroll
+        for (int u = 0; u < kFillItems; ++u) {
+            const int slot = base + u * 32 + lane;
+            int owner = 0;  // the last lane whose first item is at or before slot
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const int e = __shfl_sync(0xffffffffu, excl, owner + step);
+                if (e <= slot) owner += step;
             }
+            const int k = slot - __shfl_sync(0xffffffffu, excl, owner);
+            const uint32_t olo = __shfl_sync(0xffffffffu, mlo, owner), ohi = __shfl_sync(0xffffffffu, mhi, owner);
+            ent[u] = make_int4(__shfl_sync(0xffffffffu, lw.x, owner), __shfl_sync(0xffffffffu, lw.y, owner),
+                               __shfl_sync(0xffffffffu, lw.z, owner), __shfl_sync(0xffffffffu, lw.w, owner));
+            const int oorg = __shfl_sync(0xffffffffu, org, owner), opitch = __shfl_sync(0xffffffffu, pitch, owner);
+            const int ontx = __shfl_sync(0xffffffffu, ntx, owner);
+            tile[u] = -1;
+            if (slot < total) {
+                const int bit = select_bit((uint64_t)olo | ((uint64_t)ohi << 32), k);
+                // bit / ontx, both at most 64: (bit + 1/2) / ontx stays clear of the integers
+                const int row = (int)__fdividef((float)bit + 0.5f, (float)ontx);
+                tile[u] = oorg + row * opitch + (bit - row * ontx);
+            }
+        }
+        int64_t at[kFillItems];
+#pragma unroll
+        for (int u = 0; u < kFillItems; ++u)
+            if (tile[u] >= 0) at[u] = offsets[tile[u]] + atomicAdd(cursor + tile[u], 1);
+#pragma unroll
+        for (int u = 0; u < kFillItems; ++u)
+            if (tile[u] >= 0) {
+                if (at[u] < capacity) *reinterpret_cast<int4*>(list + at[u]) = ent[u];
+                else over = true;
+            }
+    }
+    for (unsigned big = __ballot_sync(0xffffffffu, live && !small); big != 0; big &= big - 1u) {
+        const int src = __ffs(big) - 1;
+        const int64_t oi = __shfl_sync(0xffffffffu, i, src);
+        const int ontx = __shfl_sync(0xffffffffu, ntx, src), onty = __shfl_sync(0xffffffffu, nty, src);
+        const int4 ent = make_int4(__shfl_sync(0xffffffffu, lw.x, src), __shfl_sync(0xffffffffu, lw.y, src),
+                                   __shfl_sync(0xffffffffu, lw.z, src), __shfl_sync(0xffffffffu, lw.w, src));
+        const ds_view_desc vd = views[__shfl_sync(0xffffffffu, b, src)];
+        const TriVerts v = verts[oi];
+        const int tx0 = (short)(ent.y & 0xffff) / DS_TILE, ty0 = (short)(ent.x & 0xffff) / DS_TILE;
+        for (int k = lane; k < ontx * onty; k += 32) {
+            const int ty = ty0 + k / ontx, tx = tx0 + k % ontx;
+            if (!tile_may_cover(v, vd, tx, ty)) continue;
+            const int tile = vd.tile_base + ty * vd.tiles_x + tx;
+            const int64_t at = offsets[tile] + atomicAdd(cursor + tile, 1);
+            if (at < capacity) *reinterpret_cast<int4*>(list + at) = ent;
+            else over = true;
+        }
     }
     if (over) atomicOr(status, DS_STATUS_LIST_OVERFLOW);
 }
@@ -290,31 +374,34 @@ __global__ void __launch_bounds__(kThreads) bin_fill_kernel(int B, const ds_view
 // the same slot of another lane (a shuffle).
 template <int R>
 __device__ __forceinline__ void warp_bitonic(float (&key)[R], int (&pos)[R], int lane) {
-#pragma unroll
+#pragma unroll 1
     for (int k = 2; k <= R * 32; k <<= 1) {
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j >= 32) {
+        for (int h = R / 2; h > 0; h >>= 1) {  // partners h slots apart (register indices are static)
+            if (k <= 32 * h) continue;
 #pragma unroll
-                for (int s = 0; s < R; ++s) {
-                    const int t = s ^ (j >> 5);
-                    if (t > s) {
-                        const bool up = ((s * 32 + lane) & k) == 0;  // the lower element keeps the smaller key
-                        if ((key[s] > key[t]) == up && key[s] != key[t]) {
-                            const float kk = key[s]; key[s] = key[t]; key[t] = kk;
-                            const int pp = pos[s]; pos[s] = pos[t]; pos[t] = pp;
-                        }
-                    }
+            for (int s = 0; s < R; ++s) {
+                const int t = s ^ h;
+                if (t > s) {
+                    const bool up = ((s * 32 + lane) & k) == 0;  // the lower element keeps the smaller key
+                    const float a = key[s], c = key[t];
+                    const int pa = pos[s], pc = pos[t];
+                    const bool swap = ((a > c) == up) & (a != c);  // selects, no branch
+                    key[s] = swap ? c : a; key[t] = swap ? a : c;
+                    pos[s] = swap ? pc : pa; pos[t] = swap ? pa : pc;
                 }
-            } else {
+            }
+        }
+#pragma unroll 1
+        for (int j = k > 32 ? 16 : k >> 1; j > 0; j >>= 1) {
 #pragma unroll
-                for (int s = 0; s < R; ++s) {
-                    const float ok = __shfl_xor_sync(0xffffffffu, key[s], j);
-                    const int op = __shfl_xor_sync(0xffffffffu, pos[s], j);
-                    const bool up = ((s * 32 + lane) & k) == 0, lower = (lane & j) == 0;
-                    const bool take = (lower == up) ? (ok < key[s]) : (ok > key[s]);
-                    if (take) { key[s] = ok; pos[s] = op; }
-                }
+            for (int s = 0; s < R; ++s) {
+                const float ok = __shfl_xor_sync(0xffffffffu, key[s], j);
+                const int op = __shfl_xor_sync(0xffffffffu, pos[s], j);
+                const bool up = ((s * 32 + lane) & k) == 0, lower = (lane & j) == 0;
+                const bool take = ((ok < key[s]) == (lower == up)) & (ok != key[s]);
+                key[s] = take ? ok : key[s];
+                pos[s] = take ? op : pos[s];
             }
         }
     }
@@ -341,17 +428,19 @@ __device__ __forceinline__ void sort_in_registers(const int4* __restrict__ F, in
 }
 
 // Pass 3: each tile's list ordered by zlo, from the fill pass's lists into
-// the rasterizer's (warp per tile): the (key, position) pairs are sorted by a
-// bitonic network in registers (up to 128 entries) or in shared memory (up to
-// kSortMax), and each entry is then gathered once.  Longer lists are copied
-// as they are and marked unsorted; lists cut by the capacity are not used.
+// the rasterizer's (warp per tile): the (key, position) pairs of up to kSortMax
+// entries are sorted by a bitonic network in registers, and each entry is then
+// gathered once.  Longer lists are copied as they are and marked unsorted; lists
+// cut by the capacity are not used.  A warp's own latency is the bound: the
+// network's selects have no branches and its stages are loops (with branches and
+// two smem words per pair for the long lists, the 282-entry list of 6 uneven
+// views alone took 60 us): 75 -> 24 us there, 28 -> 20 us for 8 views of 800x800,
+// 13 -> 7.6 us for one view of 1200x1200.
 __global__ void __launch_bounds__(kSortWarps * 32) sort_lists_kernel(int num_tiles,
                                                                      const int64_t* __restrict__ offsets,
                                                                      const ListEntry* __restrict__ fill,
                                                                      ListEntry* __restrict__ list, int64_t capacity,
                                                                      int* __restrict__ sorted) {
-    __shared__ float s_key[kSortWarps][kSortMax];
-    __shared__ short s_pos[kSortWarps][kSortMax];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x * kSortWarps + warp;
     if (tile >= num_tiles) return;
@@ -368,66 +457,11 @@ __global__ void __launch_bounds__(kSortWarps * 32) sort_lists_kernel(int num_til
         if (lane == 0) sorted[tile] = 0;
         return;
     }
-    if (n <= 32) {  // one entry per lane: bitonic network on (key, lane) in registers
-        int4 ent = make_int4(0, 0, 0, 0);
-        float key = INFINITY;
-        int src = lane;
-        if (lane < n) {
-            ent = F[lane];
-            key = fminf(__int_as_float(ent.z), 3.0e38f);  // real keys stay below the +inf padding
-        }
-        if (n > 1) {
-#pragma unroll
-            for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const float ok = __shfl_xor_sync(0xffffffffu, key, j);
-                    const int os = __shfl_xor_sync(0xffffffffu, src, j);
-                    // the lower lane of the pair keeps the smaller key in ascending runs
-                    const bool up = (lane & k) == 0, lower = (lane & j) == 0;
-                    const bool take = (lower == up) ? (ok < key) : (ok > key);
-                    if (take) { key = ok; src = os; }
-                }
-            }
-        }
-        const int4 out = make_int4(__shfl_sync(0xffffffffu, ent.x, src), __shfl_sync(0xffffffffu, ent.y, src),
-                                   __shfl_sync(0xffffffffu, ent.z, src), __shfl_sync(0xffffffffu, ent.w, src));
-        if (lane < n) L[lane] = out;
-        if (lane == 0) sorted[tile] = 1;
-        return;
-    }
-    if (n <= 128) {
-        if (n <= 64) sort_in_registers<2>(F, L, n, lane);
-        else sort_in_registers<4>(F, L, n, lane);
-        if (lane == 0) sorted[tile] = 1;
-        return;
-    }
-    int size = 256;
-    while (size < n) size <<= 1;
-    float* key = s_key[warp];
-    short* pos = s_pos[warp];
-    for (int i = lane; i < size; i += 32) {
-        key[i] = i < n ? fminf(__int_as_float(F[i].z), 3.0e38f) : INFINITY;  // real keys stay below the padding
-        pos[i] = (short)i;
-    }
-    __syncwarp();
-    for (int k = 2; k <= size; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = lane; i < size; i += 32) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const float a = key[i], c = key[l];
-                    const bool up = (i & k) == 0;
-                    if ((a > c) == up && a != c) {
-                        key[i] = c; key[l] = a;
-                        const short t = pos[i]; pos[i] = pos[l]; pos[l] = t;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
-    for (int i = lane; i < n; i += 32) L[i] = F[pos[i]];
+    if (n <= 32) sort_in_registers<1>(F, L, n, lane);
+    else if (n <= 64) sort_in_registers<2>(F, L, n, lane);
+    else if (n <= 128) sort_in_registers<4>(F, L, n, lane);
+    else if (n <= 256) sort_in_registers<8>(F, L, n, lane);
+    else sort_in_registers<16>(F, L, n, lane);
     if (lane == 0) sorted[tile] = 1;
 }
 
@@ -959,9 +993,12 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
     DS_CUDA(cudaMemsetAsync(w.counts, 0, (size_t)num_tiles * sizeof(int), st));
     if (!one_cta) DS_CUDA(cudaMemsetAsync(w.cursor, 0, (size_t)num_tiles * sizeof(int), st));
     const int64_t n = (int64_t)B * T;
-    if (n > 0)
-        bin_setup_kernel<<<blocks_for(n), kThreads, 0, st>>>(B, views, V, pos, T, tri, w.boxes, w.verts, w.ndc,
-                                                              w.edges, w.counts);
+    const bool narrow = n <= kBinNarrow;
+    const unsigned grid = blocks_for(narrow ? n * 4 : n);  // 8 or 32 triangles per warp
+    if (n > 0) {
+        const auto setup = narrow ? bin_setup_kernel<8> : bin_setup_kernel<32>;
+        setup<<<grid, kThreads, 0, st>>>(B, views, V, pos, T, tri, w.boxes, w.verts, w.ndc, w.edges, w.counts);
+    }
     if (one_cta) {
         scan_one_cta_kernel<<<1, kScanOneThreads, 0, st>>>(w.counts, num_tiles, w.offsets, w.cursor);
     } else {
@@ -971,10 +1008,11 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
         // offsets[num_tiles] = total number of entries
         DS_CUDA(cudaMemcpyAsync(w.offsets + num_tiles, total_dev, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
     }
-    if (n > 0)
-        bin_fill_kernel<<<blocks_for(n), kThreads, 0, st>>>(B, views, T, w.boxes, w.verts, w.ndc, w.offsets, w.cursor,
-                                                            w.fill,
-                                                            list_capacity, status);
+    if (n > 0) {
+        const auto fill = narrow ? bin_fill_kernel<8> : bin_fill_kernel<32>;
+        fill<<<grid, kThreads, 0, st>>>(B, views, T, w.boxes, w.verts, w.ndc, w.offsets, w.cursor, w.fill,
+                                        list_capacity, status);
+    }
     if (num_tiles > 0)
         sort_lists_kernel<<<(unsigned)((num_tiles + kSortWarps - 1) / kSortWarps), kSortWarps * 32, 0, st>>>(
             num_tiles, w.offsets, w.fill, w.list, list_capacity, w.sorted);
