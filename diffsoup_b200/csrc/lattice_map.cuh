@@ -39,7 +39,7 @@ struct MapTables {
 
 // Bytes of the tables: N = 3 * levels * target samples pairs, `rows` output rows.
 __host__ __device__ inline size_t map_table_bytes(int N, int rows) {
-    return ((size_t)N * 16 + (size_t)(rows + 1) * 8 + 15) & ~(size_t)15;
+    return ((size_t)N * 16 + (size_t)(rows + 1) * 8 + 127) & ~(size_t)127;
 }
 
 __device__ inline MapTables map_tables_at(unsigned char* base, int N, int rows) {

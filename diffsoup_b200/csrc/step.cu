@@ -15,6 +15,7 @@
 #include <cstdio>
 
 #include "edge_math.cuh"
+#include "lattice_map.cuh"
 #include "shade.cuh"
 #include "shade_reg.cuh"
 #include "shade_tc.cuh"
@@ -108,309 +109,260 @@ __global__ void __launch_bounds__(kPrepWarps * 32) accum_sigmoid_backward_kernel
 }
 
 // ---------------------------------------------------------------------------
-// Table-driven level accumulation.  The interpolation from the levels'
-// lattices to the target lattice is the same sparse map for every triangle,
-// so each CTA of the forward kernel builds it in shared memory (the grid is
-// one wave of persistent CTAs) and the adjoint copies the forward's: the
-// forward table lists, per
-// target sample, its (source sample, weight) pairs in level-then-corner
-// order (the summation order of accum_sigmoid_kernel), and the backward
-// table is the same map grouped by source sample, which turns the adjoint
-// into a gather without atomics.  Pairs of weight zero are left out (a
-// target sample that is a lattice vertex of a level takes one corner there):
-// about half of them, and adding 0 * x leaves a finite sum unchanged.
+// Level accumulation of the step through the map's rows (lattice_map.cuh),
+// opacity and features in one launch each way.  A group of one or two warps takes G
+// triangles at a time; a lane takes four channels of one output sample, so a row's entry and
+// one 16-byte shared load feed four products.  Features sit in the group's tile
+// as [triangle][sample][CP], opacities as [sample][triangle] (with G = 4 they
+// are one more group of four).  The sources are copied with cp.async; the adjoint
+// forms g s (1 - s) on the way in.  Only pairs of nonzero weight are used.
+// Issue slots (0.7 a cycle) and the tile's shared loads share the bound: a second
+// tile per warp for copies ahead halved the resident warps (637 us forward), one
+// triangle a warp put half of the loads on the banks of another row (493 us).
 //
-// The kernels run a warp over G = 32 / CP triangles at a time, lane (g, c)
-// taking channel c of triangle g: every lane walks the same table row, so
-// the table reads are broadcasts and the loops lane-uniform; the sources (or
-// the target gradients) of the G triangles sit in shared memory as
-// [sample][lane].  The opacities of the G triangles go through the same
-// table with lane (g, j) taking the target (or source) samples j, j + CP, ...
+// 200,000 triangles, levels 0..3, 16 channels (1.8 GB read and written forward,
+// 2.1 GB in the adjoint): forward 1014 -> 447 us, adjoint 756 -> 496 us; 60,000
+// triangles of 7 channels, levels 0..2: 50 -> 38 and 40 -> 41 us, against one
+// lane per channel with a 4-byte load and a table read per product.  Four
+// triangles interleaved in the tile instead of four channels (the layout of the
+// operators, which take any channel count) left too few warps on an SM: 1038
+// and 1673 us.
 // ---------------------------------------------------------------------------
-constexpr int kTabMax = 1024;  // (target sample, level, corner) entries
-constexpr int kTabWarps = 8;
-constexpr size_t kTabSmemMax = 100 * 1024;  // two CTAs per SM at most this size
-
-// The tables in dynamic shared memory (room for N nonzero pairs), followed
-// by each warp's staging buffer.
-struct LatticeTab {
-    int2* fent;  // per target sample (rows frow): {source sample, weight bits}
-    int* frow;   // [ST + 1]
-    int2* bent;  // per source sample (rows brow): {target sample, weight bits}
-    int* brow;   // [S + 1]
-};
-
-__host__ __device__ inline size_t lattice_tab_bytes(int N, int S, int ST) {
-    return ((size_t)N * 16 + (size_t)(S + ST + 2) * 4 + 15) & ~(size_t)15;
-}
-
-__device__ inline LatticeTab lattice_tab_at(unsigned char* base, int N, int S, int ST) {
-    LatticeTab L;
-    L.fent = reinterpret_cast<int2*>(base);
-    L.bent = reinterpret_cast<int2*>(base + (size_t)N * 8);
-    L.frow = reinterpret_cast<int*>(base + (size_t)N * 16);
-    L.brow = L.frow + ST + 1;
-    return L;
-}
-
-// Per-warp staging floats: a [rows][32] sample-by-lane buffer and the G
-// triangles' opacity rows (rows = S sources forward, ST targets backward).
-__host__ __device__ inline int tab_stage_floats(int rows, int CP) { return 32 * rows + (32 / CP) * (rows + 1); }
-
-// Exclusive prefix of rows[1..n] into rows[0..n] (rows[0] = 0), one warp.
-__device__ inline void tab_scan(int* rows, int n) {
-    const int lane = threadIdx.x & 31;
-    int carry = 0;
-    if (lane == 0) rows[0] = 0;
-    for (int d0 = 0; d0 < n; d0 += 32) {
-        const int d = d0 + lane;
-        int v = d < n ? rows[d + 1] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += u;
-        }
-        if (d < n) rows[d + 1] = carry + v;
-        carry += __shfl_sync(0xffffffffu, v, 31);
-    }
-}
-
-// Builds the tables; `scratch` holds N ints, N floats and S ints during the build.
-__device__ void build_lattice_tab(const LatticeTab& L, int lo, int hi, int ST, int S, unsigned char* scratch) {
-    const int NL = hi - lo + 1, NE = NL * 3, N = ST * NE;
-    int* fidx = reinterpret_cast<int*>(scratch);
-    float* fw = reinterpret_cast<float*>(scratch + (size_t)N * 4);
-    const float inv_r = 1.f / (float)(1u << hi);  // a power of two: x * inv_r == x / 2^hi exactly
-    for (int u = threadIdx.x; u < ST * NL; u += blockDim.x) {
-        const int k = u / NL, li = u - (u / NL) * NL, l = lo + li;
-        uint32_t x, y;
-        index_to_xy((uint32_t)k, x, y);
-        uint32_t idx[3];
-        float w[3];
-        lattice_cell(__fmul_rn((float)x, inv_r), __fmul_rn((float)y, inv_r), (uint32_t)l, idx, w);
-        uint32_t off = 0;
-        for (int m = lo; m < l; ++m) off += feats_at_level((uint32_t)m);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            fidx[k * NE + li * 3 + j] = (int)(off + idx[j]);
-            fw[k * NE + li * 3 + j] = w[j];
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < ST; k += blockDim.x) {  // forward row lengths
-        int cnt = 0;
-        for (int n = 0; n < NE; ++n) cnt += fw[k * NE + n] != 0.f;
-        L.frow[k + 1] = cnt;
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int d = threadIdx.x; d < S; d += blockDim.x) L.brow[d + 1] = 0;  // backward row lengths
-    __syncthreads();
-    for (int e = threadIdx.x; e < N; e += blockDim.x)
-        if (fw[e] != 0.f) atomicAdd(&L.brow[fidx[e] + 1], 1);
-    __syncthreads();
-    if (warp == 0) tab_scan(L.frow, ST);
-    if (warp == 1 % nw) tab_scan(L.brow, S);
-    __syncthreads();
-    for (int k = threadIdx.x; k < ST; k += blockDim.x) {  // forward rows, in (level, corner) order
-        int at = L.frow[k];
-        for (int n = 0; n < NE; ++n)
-            if (fw[k * NE + n] != 0.f) L.fent[at++] = make_int2(fidx[k * NE + n], __float_as_int(fw[k * NE + n]));
-    }
-    if (warp == nw - 1) {  // backward rows, in (target, level, corner) order: one warp walks the pairs
-        int* cursor = reinterpret_cast<int*>(fw + N);  // per source: the next free slot of its row
-        for (int d = lane; d < S; d += 32) cursor[d] = L.brow[d];
-        __syncwarp();
-        for (int e0 = 0; e0 < N; e0 += 32) {
-            const int e = e0 + lane;
-            const bool hit = e < N && fw[e] != 0.f;
-            const int d = hit ? fidx[e] : -1;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);  // the lanes with this source
-            const int leader = __ffs(peers) - 1;
-            int base = 0;
-            if (hit && lane == leader) {
-                base = cursor[d];
-                cursor[d] = base + __popc(peers);
-            }
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (hit) L.bent[base + __popc(peers & ((1u << lane) - 1u))] = make_int2(e / NE, __float_as_int(fw[e]));
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-}
+constexpr int kTabMax = 1024;  // (target sample, level, corner) pairs
 
 __device__ __forceinline__ float sigmoid_ref(float x) { return 1.f / (1.f + expf(-x)); }
 
-// 4-byte global -> shared copy that bypasses registers (cp.async), and the wait for all of a thread's.
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
+// Triangles a group takes at a time and warps of a group, by channel stride: 4
+// triangles on one warp where they have 8 channels, 2 on two warps where they
+// have 16 (their tile is too large for one tile a warp).
+template <int CP>
+constexpr int kTabGroup = CP == 8 ? 4 : 2;
+template <int CP>
+constexpr int kTabGroupWarps = CP == 8 ? 1 : 2;
+
+// Floats between the triangles of a tile: the eight lanes of a quarter warp read
+// the same sample of G triangles, so their rows must fall in different banks.
+__host__ __device__ constexpr int tab_triangle_floats(int samples, int CP) {
+    return ((samples * CP - CP + 31) / 32) * 32 + CP;
+}
+
+// Tile floats of a group: the triangles' features, then their opacities.
+__host__ __device__ constexpr int tab_tile_floats(int samples, int CP, int G) {
+    return G * tab_triangle_floats(samples, CP) + ((samples * G + 31) & ~31);
+}
+
+// Barrier of a group's lanes.
+template <int GW>
+__device__ __forceinline__ void tab_group_sync(int group) {
+    if (GW == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(GW * 32) : "memory");
+}
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem),
+                 "n"(BYTES)
                  : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+
+// Output rows of the features of G triangles and of their opacities, over the
+// group's lanes: feature(triangle, row, quad, value4), opacity(row, triangle,
+// value).
+template <int CP, int G, int GW, class Feature, class Opacity>
+__device__ __forceinline__ void tab_rows(const MapRows& m, const float* tile, int samples, int rows, Feature feature,
+                                         Opacity opacity) {
+    constexpr int Q = CP / 4;
+    const int lane = threadIdx.x % (32 * GW);
+    const int ts = tab_triangle_floats(samples, CP);
+    const float* ta = tile + G * ts;
+    const int nf = G * Q * rows;
+    // with G = 4 the opacity rows go on where the feature rows end, with the same loads
+    for (int s = lane; s < nf + (G == 4 ? rows : 0); s += 32 * GW) {
+        const bool f = G != 4 || s < nf;
+        const int q = s % Q, g = s / Q % G;
+        const int row = f ? s / (Q * G) : s - nf;
+        const float* x0 = f ? tile + g * ts + q * 4 : ta;
+        const int stride = f ? CP : 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int end = m.row[row + 1];
+#pragma unroll 2
+        for (int n = m.row[row]; n < end; ++n) {
+            const int2 e = m.ent[n];
+            const float w = __int_as_float(e.y);
+            const float4 x = *reinterpret_cast<const float4*>(x0 + e.x * stride);
+            v.x = madd(v.x, w, x.x); v.y = madd(v.y, w, x.y); v.z = madd(v.z, w, x.z); v.w = madd(v.w, w, x.w);
+        }
+        if (f) {
+            feature(g, row, q, v);
+        } else {
+            opacity(row, 0, v.x); opacity(row, 1, v.y); opacity(row, 2, v.z); opacity(row, 3, v.w);
+        }
+    }
+    if (G == 2)
+        for (int row = lane; row < rows; row += 32 * GW) {
+            float2 v = make_float2(0.f, 0.f);
+            const int end = m.row[row + 1];
+            for (int n = m.row[row]; n < end; ++n) {
+                const int2 e = m.ent[n];
+                const float w = __int_as_float(e.y);
+                const float2 x = *reinterpret_cast<const float2*>(ta + e.x * 2);
+                v.x = madd(v.x, w, x.x); v.y = madd(v.y, w, x.y);
+            }
+            opacity(row, 0, v.x); opacity(row, 1, v.y);
+        }
 }
 
 // alpha_out[t] = sigmoid(accumulate(alpha_src[t])), feat_out[t] likewise
 // per channel (+ a bf16 copy; both with the channel stride CP >= C, padding
-// channels zero).
+// channels zero).  The grid's last CTA builds the adjoint's rows meanwhile and
+// leaves them in adj_ent [N], adj_row [S + 1].
 template <int C, int CP>
-__global__ void __launch_bounds__(kTabWarps * 32) accum_tab_kernel(int T, int lo, int hi, int S, int ST,
+__global__ void __launch_bounds__(kMapWarps * 32) accum_tab_kernel(int T, int lo, int hi, int S, int ST,
                                                                    const float* __restrict__ alpha_src,
                                                                    const float* __restrict__ feat_src,
                                                                    float* __restrict__ alpha_out,
                                                                    float* __restrict__ feat_out,
                                                                    __nv_bfloat16* __restrict__ feat_bf16,
-                                                                   uint4* __restrict__ tab_out) {
-    constexpr int G = 32 / CP;
-    static_assert(CP == 8 || CP == 16, "channel stride of the accumulated tables");
-    extern __shared__ __align__(16) unsigned char tab_smem[];
+                                                                   int2* __restrict__ adj_ent, int* __restrict__ adj_row) {
+    constexpr int G = kTabGroup<CP>, GW = kTabGroupWarps<CP>, L = 32 * GW;
+    extern __shared__ __align__(16) unsigned char map_smem[];
     const int N = ST * (hi - lo + 1) * 3;
-    const size_t tab_bytes = lattice_tab_bytes(N, S, ST);
-    const LatticeTab L = lattice_tab_at(tab_smem, N, S, ST);
-    build_lattice_tab(L, lo, hi, ST, S, tab_smem + tab_bytes);  // the scratch is the staging area
-    if (blockIdx.x == 0) {  // the tables for the adjoint kernel of this step
-        const uint4* src = reinterpret_cast<const uint4*>(tab_smem);
-        for (int i = threadIdx.x; i < (int)(tab_bytes / 16); i += blockDim.x) tab_out[i] = src[i];
+    if (blockIdx.x == gridDim.x - 1) {
+        const MapTables a = map_tables_at(map_smem, N, S);
+        build_adjoint_rows(a, lo, hi, hi, ST, S);
+        for (int i = threadIdx.x; i < N; i += blockDim.x) adj_ent[i] = a.nonzero.ent[i];
+        for (int i = threadIdx.x; i <= S; i += blockDim.x) adj_row[i] = a.nonzero.row[i];
+        return;
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / CP, c = lane % CP;
-    const int M = S;
-    float* sf = reinterpret_cast<float*>(tab_smem + tab_bytes) + (size_t)warp * tab_stage_floats(M, CP);
-    float* sa = sf + 32 * M;  // [G][M + 1]
-    for (int t0 = (blockIdx.x * kTabWarps + warp) * G; t0 < T; t0 += gridDim.x * kTabWarps * G) {
-        const int t = t0 + g;
-        const bool tv = t < T;
-        // every sample copied without registers (cp.async), then one wait: one round trip a pass
-        for (int s = 0; s < S; ++s) {
-            float* dst = sf + s * 32 + lane;
-            if (tv && c < C) cp_async4(dst, feat_src + ((size_t)t * S + s) * C + c);
-            else *dst = 0.f;
-        }
-        for (int i = lane; i < G * S; i += 32) {
-            const int gi = i / S;
-            float* dst = sa + gi * (M + 1) + (i - gi * S);
-            if (t0 + gi < T) cp_async4(dst, alpha_src + (size_t)t0 * S + i);
-            else *dst = 0.f;
-        }
-        cp_async_wait_all();
-        __syncwarp();
-        // opacity: lane (g, j) takes targets j, j + CP, ...
-        for (int k = c; k < ST; k += CP) {
-            float acc = 0.f;
-            for (int n = L.frow[k]; n < L.frow[k + 1]; ++n) {
-                const int2 e = L.fent[n];
-                acc = madd(acc, __int_as_float(e.y), sa[g * (M + 1) + e.x]);
+    const MapTables m = map_tables_at(map_smem, N, ST);
+    const int group = (threadIdx.x >> 5) / GW, lane = threadIdx.x % L;
+    const int ts = tab_triangle_floats(S, CP), tf = tab_tile_floats(S, CP, G);
+    float* tile = reinterpret_cast<float*>(map_smem + map_table_bytes(N, ST > S ? ST : S)) + (size_t)group * tf;
+    if (C < CP)
+        for (int i = lane; i < tf; i += L) tile[i] = 0.f;  // the padding channels stay zero
+    tab_group_sync<GW>(group);
+    const bool wide = C % 4 == 0 && ((uintptr_t)feat_src & 15) == 0;
+    auto stage = [&](int64_t t) {
+        for (int g = 0; g < G && t + g < T; ++g) {
+            const float* fs = feat_src + (size_t)(t + g) * S * C;
+            float* dst = tile + g * ts;
+            if (wide) {
+                for (int e = lane; e < S * (C / 4); e += L) cp_async<16>(dst + e * 4, fs + e * 4);
+            } else {
+                for (int e = lane; e < S * C; e += L) cp_async<4>(dst + (C == CP ? e : e / C * CP + e % C), fs + e);
             }
-            if (tv) alpha_out[(size_t)t * ST + k] = sigmoid_ref(acc);
+            for (int d = lane; d < S; d += L) cp_async<4>(tile + G * ts + d * G + g, alpha_src + (size_t)(t + g) * S + d);
         }
-        // features: lane (g, c) takes channel c of every target
-        for (int k = 0; k < ST; ++k) {
-            float acc = 0.f;
-#pragma unroll 4
-            for (int n = L.frow[k]; n < L.frow[k + 1]; ++n) {
-                const int2 e = L.fent[n];
-                acc = madd(acc, __int_as_float(e.y), sf[e.x * 32 + lane]);
-            }
-            const float v = c < C ? sigmoid_ref(acc) : 0.f;
-            if (tv) {
-                feat_out[((size_t)t * ST + k) * CP + c] = v;
-                feat_bf16[((size_t)t * ST + k) * CP + c] = __float2bfloat16_rn(v);
-            }
-        }
-        __syncwarp();
+    };
+    const int64_t step = (int64_t)(gridDim.x - 1) * (kMapWarps / GW) * G;
+    int64_t t = ((int64_t)blockIdx.x * (kMapWarps / GW) + group) * G;
+    stage(t);
+    build_forward_rows(m, lo, hi, hi, ST);
+    for (; t < T; t += step) {
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        tab_group_sync<GW>(group);
+        tab_rows<CP, G, GW>(
+            m.nonzero, tile, S, ST,
+            [&](int g, int row, int q, float4 v) {
+                if (t + g >= T) return;
+                float4 y = make_float4(sigmoid_ref(v.x), sigmoid_ref(v.y), sigmoid_ref(v.z), sigmoid_ref(v.w));
+                if (C == 7 && q == 1) y.w = 0.f;
+                const size_t o = ((size_t)(t + g) * ST + row) * CP + q * 4;
+                *reinterpret_cast<float4*>(feat_out + o) = y;
+                const __nv_bfloat162 a = __floats2bfloat162_rn(y.x, y.y), c = __floats2bfloat162_rn(y.z, y.w);
+                *reinterpret_cast<uint2*>(feat_bf16 + o) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
+            },
+            [&](int row, int g, float v) {
+                if (t + g < T) alpha_out[(size_t)(t + g) * ST + row] = sigmoid_ref(v);
+            });
+        tab_group_sync<GW>(group);
+        stage(t + step);
     }
 }
 
 // Adjoint of accum_tab_kernel: grad_src[t][d] = sum over the targets k that
 // read d of w * grad_out[t][k] * s (1 - s); a gather, written once.  feat_sig and
-// feat_grad have the channel stride CP, feat_src_grad the stride C.
+// feat_grad have the channel stride CP (padding channels zero), feat_src_grad
+// the stride C.
 template <int C, int CP>
-__global__ void __launch_bounds__(kTabWarps * 32) accum_tab_backward_kernel(
+__global__ void __launch_bounds__(kMapWarps * 32) accum_tab_backward_kernel(
     int T, int lo, int hi, int S, int ST, const float* __restrict__ alpha_sig, const float* __restrict__ alpha_grad,
     const float* __restrict__ feat_sig, const float* __restrict__ feat_grad, float* __restrict__ alpha_src_grad,
-    float* __restrict__ feat_src_grad, const uint4* __restrict__ tab_in) {
-    constexpr int G = 32 / CP;
-    extern __shared__ __align__(16) unsigned char tab_smem[];
+    float* __restrict__ feat_src_grad, const int2* __restrict__ adj_ent, const int* __restrict__ adj_row) {
+    constexpr int G = kTabGroup<CP>, GW = kTabGroupWarps<CP>, L = 32 * GW, Q = CP / 4;
+    extern __shared__ __align__(16) unsigned char map_smem[];
     const int N = ST * (hi - lo + 1) * 3;
-    const size_t tab_bytes = lattice_tab_bytes(N, S, ST);
-    const LatticeTab L = lattice_tab_at(tab_smem, N, S, ST);
-    {
-        uint4* dst = reinterpret_cast<uint4*>(tab_smem);
-        for (int i = threadIdx.x; i < (int)(tab_bytes / 16); i += blockDim.x) dst[i] = tab_in[i];
-        __syncthreads();
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / CP, c = lane % CP;
-    const int M = ST;
-    float* gf = reinterpret_cast<float*>(tab_smem + tab_bytes) + (size_t)warp * tab_stage_floats(M, CP);
-    float* ga = gf + 32 * M;  // [G][M + 1]
-    for (int t0 = (blockIdx.x * kTabWarps + warp) * G; t0 < T; t0 += gridDim.x * kTabWarps * G) {
-        const int t = t0 + g;
-        const bool tv = t < T;
-        // sixteen (sigmoid, gradient) pairs in flight per lane before their stores
-        for (int k0 = 0; k0 < ST; k0 += 16) {
-            float sg[16], gr[16];
+    MapRows m;
+    m.ent = reinterpret_cast<int2*>(map_smem);
+    m.row = reinterpret_cast<int*>(m.ent + N);
+    const int group = (threadIdx.x >> 5) / GW, lane = threadIdx.x % L;
+    const int ts = tab_triangle_floats(ST, CP);
+    float* tile = reinterpret_cast<float*>(map_smem + (((size_t)N * 8 + (size_t)(S + 1) * 4 + 127) & ~(size_t)127)) +
+                  (size_t)group * tab_tile_floats(ST, CP, G);
+    for (int i = threadIdx.x; i <= S; i += blockDim.x) m.row[i] = adj_row[i];
+    for (int i = threadIdx.x; i < adj_row[S]; i += blockDim.x) m.ent[i] = adj_ent[i];
+    __syncthreads();
+    const bool wide = C % 4 == 0 && ((uintptr_t)feat_src_grad & 15) == 0;
+    const int64_t step = (int64_t)gridDim.x * (kMapWarps / GW) * G;
+    for (int64_t t = ((int64_t)blockIdx.x * (kMapWarps / GW) + group) * G; t < T; t += step) {
+        for (int g = 0; g < G && t + g < T; ++g) {
+            const float4* sp = reinterpret_cast<const float4*>(feat_sig + (size_t)(t + g) * ST * CP);
+            const float4* gp = reinterpret_cast<const float4*>(feat_grad + (size_t)(t + g) * ST * CP);
+            for (int e0 = lane; e0 < ST * Q; e0 += 3 * L) {  // three (sigmoid, gradient) pairs in flight
+                float4 y[3], v[3];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const bool in = k0 + j < ST && tv && c < C;
-                const size_t o = ((size_t)t * ST + k0 + j) * CP + c;
-                sg[j] = in ? __ldg(feat_sig + o) : 0.f;
-                gr[j] = in ? __ldg(feat_grad + o) : 0.f;
+                for (int u = 0; u < 3; ++u)
+                    if (e0 + L * u < ST * Q) { y[u] = __ldg(sp + e0 + L * u); v[u] = __ldg(gp + e0 + L * u); }
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (e0 + L * u < ST * Q) {
+                        v[u].x = v[u].x * y[u].x * (1.f - y[u].x); v[u].y = v[u].y * y[u].y * (1.f - y[u].y);
+                        v[u].z = v[u].z * y[u].z * (1.f - y[u].z); v[u].w = v[u].w * y[u].w * (1.f - y[u].w);
+                        *reinterpret_cast<float4*>(tile + g * ts + (e0 + L * u) * 4) = v[u];
+                    }
             }
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (k0 + j < ST) gf[(k0 + j) * 32 + lane] = gr[j] * sg[j] * (1.f - sg[j]);
-        }
-        for (int i0 = 0; i0 < G * ST; i0 += 128) {
-            float sg[4], gr[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = i0 + j * 32 + lane, gi = i / ST;
-                const bool in = i < G * ST && t0 + gi < T;
-                sg[j] = in ? __ldg(alpha_sig + (size_t)t0 * ST + i) : 0.f;
-                gr[j] = in ? __ldg(alpha_grad + (size_t)t0 * ST + i) : 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = i0 + j * 32 + lane, gi = i / ST;
-                if (i < G * ST) ga[gi * (M + 1) + (i - gi * ST)] = gr[j] * sg[j] * (1.f - sg[j]);
+            for (int k = lane; k < ST; k += L) {
+                const size_t o = (size_t)(t + g) * ST + k;
+                const float y = __ldg(alpha_sig + o);
+                tile[G * ts + k * G + g] = __ldg(alpha_grad + o) * y * (1.f - y);
             }
         }
-        __syncwarp();
-        for (int d = c; d < S; d += CP) {  // opacity: lane (g, j) takes sources j, j + CP, ...
-            float v = 0.f;
-            for (int n = L.brow[d]; n < L.brow[d + 1]; ++n) {
-                const int2 e = L.bent[n];
-                v = fmaf(__int_as_float(e.y), ga[g * (M + 1) + e.x], v);
-            }
-            if (tv) alpha_src_grad[(size_t)t * S + d] = v;
-        }
-        for (int d = 0; d < S; ++d) {  // features: lane (g, c) takes channel c of every source
-            float v = 0.f;
-#pragma unroll 4
-            for (int n = L.brow[d]; n < L.brow[d + 1]; ++n) {
-                const int2 e = L.bent[n];
-                v = fmaf(__int_as_float(e.y), gf[e.x * 32 + lane], v);
-            }
-            if (tv && c < C) feat_src_grad[((size_t)t * S + d) * C + c] = v;
-        }
-        __syncwarp();
+        tab_group_sync<GW>(group);
+        tab_rows<CP, G, GW>(
+            m, tile, ST, S,
+            [&](int g, int row, int q, float4 v) {
+                if (t + g >= T) return;
+                float* o = feat_src_grad + ((size_t)(t + g) * S + row) * C + q * 4;
+                if (wide) {
+                    *reinterpret_cast<float4*>(o) = v;
+                    return;
+                }
+                o[0] = v.x; o[1] = v.y; o[2] = v.z;
+                if (C % 4 == 0 || q < Q - 1) o[3] = v.w;
+            },
+            [&](int row, int g, float v) {
+                if (t + g < T) alpha_src_grad[(size_t)(t + g) * S + row] = v;
+            });
+        tab_group_sync<GW>(group);
     }
 }
 
-// Dynamic shared memory of the table kernels: tables + per-warp staging of
-// the sources (forward) or of the
-// target gradients (backward).
-static size_t lattice_tab_smem(int lo, int hi, int S, int ST, int CP, bool backward) {
+// Dynamic shared memory of the table kernels: rows and each group's tile.
+template <int CP>
+static size_t lattice_tab_smem(int lo, int hi, int S, int ST, bool backward) {
     const int N = ST * (hi - lo + 1) * 3;
-    return lattice_tab_bytes(N, S, ST) + (size_t)kTabWarps * tab_stage_floats(backward ? ST : S, CP) * 4;
+    const size_t tables = backward ? (((size_t)N * 8 + (size_t)(S + 1) * 4 + 127) & ~(size_t)127)
+                                   : map_table_bytes(N, ST > S ? ST : S);
+    return tables + (size_t)(kMapWarps / kTabGroupWarps<CP>) * tab_tile_floats(backward ? ST : S, CP, kTabGroup<CP>) *
+                        sizeof(float);
 }
 
-// Whether the table kernels cover this configuration.
+// Whether the table kernels cover this configuration (two CTAs per SM).
 static bool lattice_tab_fits(int lo, int hi, int S, int ST, int CP) {
-    return ST * (hi - lo + 1) * 3 <= kTabMax && (CP == 8 || CP == 16) &&
-           lattice_tab_smem(lo, hi, S, ST, CP, false) <= kTabSmemMax;
+    if (ST * (hi - lo + 1) * 3 > kTabMax) return false;
+    return (CP == 8 && lattice_tab_smem<8>(lo, hi, S, ST, false) <= 110 * 1024) ||
+           (CP == 16 && lattice_tab_smem<16>(lo, hi, S, ST, false) <= 110 * 1024);
 }
 
 // The table kernels' dynamic shared memory above the 48 KB default, and
@@ -422,7 +374,7 @@ static int tab_smem_attr(size_t smem, int* per_sm = nullptr) {
     static int fit = 1;
     if (smem != set) {
         DS_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, Kernel, kTabWarps * 32, smem));
+        DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, Kernel, kMapWarps * 32, smem));
         if (fit < 1) fit = 1;
         set = smem;
     }
@@ -733,7 +685,8 @@ struct StepWs {
     float* color;
     float* grad_color;
     float* l1;
-    uint4* tab;         // lattice tables of the level accumulation, from its forward kernel
+    int2* adj_ent;      // rows of the level accumulation's adjoint, left by its forward kernel
+    int* adj_row;
     double* grad_pos;
     float* grad_alpha_acc;
     float* grad_feat_acc;
@@ -774,9 +727,10 @@ static StepWs carve_step(void* ws, const ds_step_config& c, int num_tiles, int64
     w.color = reinterpret_cast<float*>(base + o); o += al((size_t)P * 12);
     w.grad_color = reinterpret_cast<float*>(base + o); o += al((size_t)P * 12);
     w.l1 = reinterpret_cast<float*>(base + o); o += al((size_t)P * 4);
-    w.tab = reinterpret_cast<uint4*>(base + o);
-    o += al(lattice_tab_bytes(ST * (c.max_level - c.min_level + 1) * 3,
-                              (int)total_feats((uint32_t)c.min_level, (uint32_t)c.max_level), ST));
+    w.adj_ent = reinterpret_cast<int2*>(base + o);
+    o += al((size_t)ST * (c.max_level - c.min_level + 1) * 3 * sizeof(int2));
+    w.adj_row = reinterpret_cast<int*>(base + o);
+    o += al((size_t)(total_feats((uint32_t)c.min_level, (uint32_t)c.max_level) + 1) * sizeof(int));
     // zeroed together each step: grad_pos .. loss_sum
     w.grad_pos = reinterpret_cast<double*>(base + o); o += al((size_t)c.B * c.V * 32);
     w.grad_alpha_acc = reinterpret_cast<float*>(base + o); o += al((size_t)c.T * ST * 4);
@@ -925,27 +879,27 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
     // prep: opacity and feature accumulation + sigmoid (side), projection (st)
     const unsigned tb = (unsigned)((c.T + kPrepWarps - 1) / kPrepWarps);
     const bool tab = lattice_tab_fits(c.min_level, c.max_level, S, ST, CP);
-    const size_t tsm = lattice_tab_smem(c.min_level, c.max_level, S, ST, CP, false);
-    const size_t tsm_bwd = lattice_tab_smem(c.min_level, c.max_level, S, ST, CP, true);
-    const int64_t tw = ((int64_t)c.T + (32 / CP) * kTabWarps - 1) / ((32 / CP) * kTabWarps);  // CTAs of 32/CP triangles a warp
-    const int64_t nsm = sm_count();
-    // the adjoint: persistent CTAs, each copying the forward's tables once
-    const unsigned tgrid_bwd = (unsigned)(tw < nsm * 8 ? tw : nsm * 8);
-    if (c.T > 0 && tab) {
-#define DSB_ACCUM_TAB(CC, CPP)                                                                                     \
+    // one wave of persistent CTAs, each holding the rows once (EXTRA: the forward's CTA for the adjoint's rows)
+#define DSB_TAB(KERNEL, BWD, EXTRA, CC, CPP, STREAM, ...)                                                          \
     do {                                                                                                           \
-        int per_sm = 1;                                                                                            \
-        if ((rc = tab_smem_attr<accum_tab_kernel<CC, CPP>>(tsm, &per_sm))) return rc;                              \
-        /* one wave of persistent CTAs, each building the tables once */                                           \
-        const unsigned tgrid = (unsigned)(tw < nsm * per_sm ? tw : nsm * per_sm);                                  \
-        accum_tab_kernel<CC, CPP><<<tgrid, kTabWarps * 32, tsm, sst>>>(c.T, c.min_level, c.max_level, S, ST,       \
-                                                                       alpha_src, feat_src, w.alpha_acc,           \
-                                                                       w.feat_acc, w.feat_bf16, w.tab);            \
+        const size_t tsm = lattice_tab_smem<CPP>(c.min_level, c.max_level, S, ST, BWD);                            \
+        int per_sm = 1, trc = tab_smem_attr<KERNEL<CC, CPP>>(tsm, &per_sm);                                        \
+        if (trc) return trc;                                                                                       \
+        const int per = kTabGroup<CPP> * (kMapWarps / kTabGroupWarps<CPP>); /* triangles of a CTA's pass */        \
+        const int64_t want = ((int64_t)c.T + per - 1) / per;                                                       \
+        const int64_t wave = (int64_t)sm_count() * per_sm - EXTRA;                                                 \
+        KERNEL<CC, CPP><<<(unsigned)((want < wave ? want : wave) + EXTRA), kMapWarps * 32, tsm, STREAM>>>(         \
+            c.T, c.min_level, c.max_level, S, ST, __VA_ARGS__);                                                    \
     } while (0)
-        if (c.C == 8) DSB_ACCUM_TAB(8, 8);
-        else if (c.C == 7) DSB_ACCUM_TAB(7, 8);
-        else DSB_ACCUM_TAB(16, 16);
-#undef DSB_ACCUM_TAB
+#define DSB_TAB_C(KERNEL, BWD, EXTRA, STREAM, ...)                                                                 \
+    do {                                                                                                           \
+        if (c.C == 8) DSB_TAB(KERNEL, BWD, EXTRA, 8, 8, STREAM, __VA_ARGS__);                                      \
+        else if (c.C == 7) DSB_TAB(KERNEL, BWD, EXTRA, 7, 8, STREAM, __VA_ARGS__);                                 \
+        else DSB_TAB(KERNEL, BWD, EXTRA, 16, 16, STREAM, __VA_ARGS__);                                             \
+    } while (0)
+    if (c.T > 0 && tab) {
+        DSB_TAB_C(accum_tab_kernel, false, 1, sst, alpha_src, feat_src, w.alpha_acc, w.feat_acc, w.feat_bf16,
+                  w.adj_ent, w.adj_row);
     } else if (c.T > 0) {
         accum_sigmoid_kernel<false><<<tb, kPrepWarps * 32, 0, sst>>>(c.T, c.min_level, c.max_level, c.max_level, S, ST,
                                                                     1, 1, alpha_src, w.alpha_acc, nullptr);
@@ -995,19 +949,9 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
     // vertex gradients, so with a side stream they run there after the opacity pass, beside the edge
     // gradients
     auto accum_backward = [&](cudaStream_t s) -> int {
-        int r = DS_OK;
         if (c.T > 0 && tab) {
-#define DSB_ACCUM_TAB_BWD(CC, CPP)                                                                                 \
-    do {                                                                                                           \
-        if ((r = tab_smem_attr<accum_tab_backward_kernel<CC, CPP>>(tsm_bwd))) return r;                            \
-        accum_tab_backward_kernel<CC, CPP><<<tgrid_bwd, kTabWarps * 32, tsm_bwd, s>>>(                             \
-            c.T, c.min_level, c.max_level, S, ST, w.alpha_acc, w.grad_alpha_acc, w.feat_acc, w.grad_feat_acc,      \
-            grad_alpha_src, grad_feat_src, w.tab);                                                                 \
-    } while (0)
-            if (c.C == 8) DSB_ACCUM_TAB_BWD(8, 8);
-            else if (c.C == 7) DSB_ACCUM_TAB_BWD(7, 8);
-            else DSB_ACCUM_TAB_BWD(16, 16);
-#undef DSB_ACCUM_TAB_BWD
+            DSB_TAB_C(accum_tab_backward_kernel, true, 0, s, w.alpha_acc, w.grad_alpha_acc, w.feat_acc, w.grad_feat_acc,
+                      grad_alpha_src, grad_feat_src, w.adj_ent, w.adj_row);
         } else if (c.T > 0) {
             accum_sigmoid_backward_kernel<<<tb, kPrepWarps * 32, 0, s>>>(c.T, c.min_level, c.max_level, c.max_level,
                                                                          S, ST, 1, 1, w.alpha_acc, w.grad_alpha_acc,
@@ -1016,8 +960,10 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
                                                                          S, ST, c.C, CP, w.feat_acc,
                                                                          w.grad_feat_acc, grad_feat_src);
         }
-        return r;
+        return DS_OK;
     };
+#undef DSB_TAB_C
+#undef DSB_TAB
 
     // opacity auxiliary gradient (scaled by 1/numel(colour), rasterize.py:183-195), on the side
     // stream beside the edge gradients
