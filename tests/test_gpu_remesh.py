@@ -166,3 +166,27 @@ def test_core_bindings_take_numpy():
     valid = np.ones(sc.T, np.int32)
     got = _core.split_triangle_soup_clip(sc.mvps()[0], sc.verts, sc.tri, valid, -1, 0.02, 400 / 300)
     _equal(got, R.restated_split(sc.verts, sc.tri, 0.02, mvp=sc.mvps()[0], valid=valid, aspect_wh=400 / 300))
+
+
+@pytest.mark.parametrize("mode,T,cut", [("world", 1, 0.02), ("world", 200, 0.3), ("world", 200, 0.06),
+                                        ("world", 4000, 0.1), ("clip", 300, 0.05), ("clip", 300, 0.004),
+                                        ("clip", 5000, 0.02)])
+def test_split_budget_finds_the_threshold(mode, T, cut):
+    """A budget of exactly the splits that a threshold makes gives the threshold's arrays, with no floor, with a
+    floor below the cut-off (in its octave and some octaves down) and, one split short, one split fewer."""
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(DEV)  # noqa: E731
+    if mode == "world":
+        v, f = _soup(T, seed=T)
+        args, split = (t(v), t(f)), remesh.split_triangle_soup
+        want = _np(remesh.split_triangle_soup_until(*args, cut))
+    else:
+        sc = scenes.make_scene(2, seed=T, num_tris=T, num_views=1, resolution=(600, 800), with_targets=False)
+        valid = (np.random.default_rng(5).random(sc.T) < 0.8).astype(np.int32)
+        args, split = ((600, 800), t(sc.mvps()[0]), t(sc.verts), t(sc.tri), t(valid)), remesh.split_triangle_soup_clip
+        want = _np(remesh.split_triangle_soup_clip_until(*args, cut))
+    K = want[1].shape[0] - T
+    assert K > 0
+    for floor in (0.0, 0.95 * cut, 0.6 * cut):
+        _equal(_np(split(*args, K, floor)), want)
+    if K > 1:
+        assert split(*args, K - 1, 0.0)[1].shape[0] == T + K - 1
