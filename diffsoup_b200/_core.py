@@ -58,11 +58,14 @@ _sig("ds_depth_test", _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp
 _sig("ds_backward_edge_grad", _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp)
 _sig("ds_backward_opacity_aux_loss", _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _vp)
 _sig("ds_encode_view_dir_sh2", _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp)
+_sig("ds_encode_view_dir_sh2_set", _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp)
+_sig("ds_encode_view_dir_set", _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp)
 _sig("ds_encode_view_dir", _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp)
 _sig("ds_count_triangle_ids", _i32, _i64, _vp, _i32, _vp, _vp, _vp)
 _sig("ds_multires_triangle_alpha", _i32, _i32, _vp, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_backward_multires_triangle_alpha", _i32, _i32, _vp, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_multires_triangle_color", _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
+_sig("ds_multires_triangle_color_set", _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_backward_multires_triangle_color", _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_accumulate_to_level_forward", _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
 _sig("ds_accumulate_to_level_backward_set", _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp)
@@ -216,6 +219,20 @@ def multires_triangle_color(rast, min_level: int, max_level: int, features, out)
     B, H, W, _ = rast.shape
     check(_lib.ds_multires_triangle_color(B, H, W, ptr(rast), min_level, max_level, features.shape[1],
                                           features.shape[2], ptr(features), ptr(out), stream()))
+
+
+def multires_triangle_color_set(rast, min_level: int, max_level: int, features, out) -> None:
+    """multires_triangle_color into an uninitialised buffer (every pixel written)."""
+    B, H, W, _ = rast.shape
+    check(_lib.ds_multires_triangle_color_set(B, H, W, ptr(rast), min_level, max_level, features.shape[1],
+                                              features.shape[2], ptr(features), ptr(out), stream()))
+
+
+def encode_view_set(rast, inv_mvp, encoding) -> None:
+    """encode_view_dir_sh2 (9 channels) or encode_view_dir (3) into an uninitialised buffer."""
+    B, H, W, _ = rast.shape
+    f = _lib.ds_encode_view_dir_sh2_set if encoding.shape[-1] == 9 else _lib.ds_encode_view_dir_set
+    check(f(B, H, W, ptr(rast), ptr(inv_mvp), ptr(encoding), stream()))
 
 
 def backward_multires_triangle_color(rast, min_level: int, max_level: int, grad_features, grad_out) -> None:

@@ -144,8 +144,8 @@ class _MultiresTriangleColorFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, rast, min_level, max_level, feat):
         B, H, W, _ = rast.shape
-        out = torch.zeros((B, H, W, feat.shape[2]), dtype=torch.float32, device=rast.device)
-        _core.multires_triangle_color(rast, min_level, max_level, feat, out)
+        out = torch.empty((B, H, W, feat.shape[2]), dtype=torch.float32, device=rast.device)
+        _core.multires_triangle_color_set(rast, min_level, max_level, feat, out)
         ctx.save_for_backward(rast)
         ctx.levels = (min_level, max_level)
         ctx.feat_shape = tuple(feat.shape)

@@ -159,8 +159,8 @@ def encode_view_dir_sh2(rast, inv_mvp) -> torch.Tensor:
     assert rast.shape == (B, H, W, 4) and rast.is_contiguous() and rast.dtype == torch.float32
     assert inv_mvp.shape == (B, 4, 4) and inv_mvp.is_contiguous() and inv_mvp.dtype == torch.float32
     assert rast.is_cuda and inv_mvp.device == dev
-    enc = torch.zeros(B, H, W, 9, dtype=torch.float32, device=dev)
-    _core.encode_view_dir_sh2(rast, inv_mvp, enc)
+    enc = torch.empty(B, H, W, 9, dtype=torch.float32, device=dev)
+    _core.encode_view_set(rast, inv_mvp, enc)
     return enc
 
 
@@ -173,8 +173,8 @@ def encode_view_dir(rast, inv_mvp) -> torch.Tensor:
     assert rast.shape == (B, H, W, 4) and rast.is_contiguous() and rast.dtype == torch.float32
     assert inv_mvp.shape == (B, 4, 4) and inv_mvp.is_contiguous() and inv_mvp.dtype == torch.float32
     assert rast.is_cuda and inv_mvp.device == dev
-    enc = torch.zeros(B, H, W, 3, dtype=torch.float32, device=dev)
-    _core.encode_view_dir(rast, inv_mvp, enc)
+    enc = torch.empty(B, H, W, 3, dtype=torch.float32, device=dev)
+    _core.encode_view_set(rast, inv_mvp, enc)
     return enc
 
 

@@ -114,6 +114,13 @@ int ds_backward_opacity_aux_loss(int B, int H, int W, int C, const float* color,
 int ds_encode_view_dir_sh2(int B, int H, int W, const float* rast, const float* inv_mvp, float* encoding,
                            ds_stream_t stream);
 
+/* The same encoding with every pixel written (background pixels zero; no
+ * zeroed buffer needed): 9 coefficients, or the raw direction (3). */
+int ds_encode_view_dir_sh2_set(int B, int H, int W, const float* rast, const float* inv_mvp, float* encoding,
+                               ds_stream_t stream);
+int ds_encode_view_dir_set(int B, int H, int W, const float* rast, const float* inv_mvp, float* encoding,
+                           ds_stream_t stream);
+
 /* replaces _core.multires_triangle_alpha (src/main.cpp:174-191, multires.cu:130-176).
  * S must equal the lattice size of levels [min_level, max_level]. */
 int ds_multires_triangle_alpha(int num_frags, const float* frag_attrs, int min_level, int max_level, int S,
@@ -129,6 +136,11 @@ int ds_backward_multires_triangle_alpha(int num_frags, const float* frag_attrs, 
  * out [B,H,W,C] accumulates (the reference zero-initialises it). */
 int ds_multires_triangle_color(int B, int H, int W, const float* rast, int min_level, int max_level, int S, int C,
                                const float* features, float* out, ds_stream_t stream);
+
+/* The same interpolation with every pixel of out [B,H,W,C] written (background
+ * pixels zero; no zeroed buffer needed). */
+int ds_multires_triangle_color_set(int B, int H, int W, const float* rast, int min_level, int max_level, int S, int C,
+                                   const float* features, float* out, ds_stream_t stream);
 
 /* replaces _core.backward_multires_triangle_color (src/main.cpp:234-254,
  * multires.cu:268-311).  grad_features [T,S,C] accumulates. */
