@@ -4,8 +4,9 @@
 (python/diffsoup/optimize.py:7-68: VectorAdam(params, lr=1e-3,
 betas=(0.9, 0.999)), step()) and `Adam` that of torch.optim.Adam as
 examples/02_synthetic.py:310-315 uses it (lr, betas, eps; no weight decay or
-amsgrad).  Each parameter is updated by one kernel of libdiffsoup_b200.so
-(ds_vector_adam_step / ds_adam_step) on torch's current stream.  The step
+amsgrad).  The parameters are updated by kernels of libdiffsoup_b200.so
+(ds_vector_adam_step per parameter, ds_adam_step_multi per group) on torch's
+current stream.  The step
 count is a device int32 in the parameter's state (state["step"]), advanced by
 the kernel, so an update can be captured in a CUDA graph together with the
 training step; the reference keeps it as a Python int.
@@ -23,6 +24,8 @@ _L = _core.lib
 _L.ds_adam_step.restype = C.c_int
 _L.ds_adam_step.argtypes = [C.c_void_p] * 4 + [C.c_int64, C.c_double, C.c_double, C.c_double, C.c_double,
                                                C.c_void_p, C.c_void_p]
+_L.ds_adam_step_multi.restype = C.c_int
+_L.ds_adam_step_multi.argtypes = [C.c_int] + [C.c_void_p] * 6 + [C.c_double] * 4 + [C.c_void_p]
 _L.ds_vector_adam_step.restype = C.c_int
 _L.ds_vector_adam_step.argtypes = [C.c_void_p] * 4 + [C.c_int64, C.c_int, C.c_double, C.c_double, C.c_double,
                                                       C.c_void_p, C.c_void_p]
@@ -68,7 +71,7 @@ class VectorAdam(torch.optim.Optimizer):
 
 class Adam(torch.optim.Optimizer):
     """torch.optim.Adam's update (no weight decay, no amsgrad) as one fused
-    kernel per parameter."""
+    launch per parameter group."""
 
     def __init__(self, params, lr=1e-3, betas=(0.9, 0.999), eps=1e-8):
         defaults = dict(lr=lr, betas=betas, eps=eps)
@@ -83,6 +86,7 @@ class Adam(torch.optim.Optimizer):
         for group in self.param_groups:
             lr, eps = group["lr"], group["eps"]
             b1, b2 = group["betas"]
+            rows = []  # (param, grad, exp_avg, exp_avg_sq, elements, step) of the group's one launch
             for p in group["params"]:
                 if p.grad is None:
                     continue
@@ -93,7 +97,10 @@ class Adam(torch.optim.Optimizer):
                     state["step"] = torch.zeros(1, dtype=torch.int32, device=p.device)
                     state["exp_avg"] = torch.zeros_like(p)
                     state["exp_avg_sq"] = torch.zeros_like(p)
-                _core.check(_L.ds_adam_step(_core.ptr(p), _core.ptr(g), _core.ptr(state["exp_avg"]),
-                                            _core.ptr(state["exp_avg_sq"]), p.numel(), lr, b1, b2, eps,
-                                            _core.ptr(state["step"]), _core.stream()))
+                rows.append((p.data_ptr(), g.data_ptr(), state["exp_avg"].data_ptr(), state["exp_avg_sq"].data_ptr(),
+                             p.numel(), state["step"].data_ptr()))
+            if rows:
+                n = len(rows)
+                cols = [(C.c_int64 * n)(*col) for col in zip(*rows)]
+                _core.check(_L.ds_adam_step_multi(n, *cols, lr, b1, b2, eps, _core.stream()))
         return loss

@@ -358,6 +358,13 @@ int ds_count_triangle_ids(int64_t num_pixels, const float* rast, int num_tris, i
 int ds_adam_step(float* param, const float* grad, float* exp_avg, float* exp_avg_sq, int64_t n, double lr,
                  double beta1, double beta2, double eps, int* step, ds_stream_t stream);
 
+/* The same update of `count` parameters with common hyperparameters, in one
+ * launch per 32 of them; the arrays (host memory) hold each parameter's device
+ * pointers and element count. */
+int ds_adam_step_multi(int count, float* const* params_host, const float* const* grads_host,
+                       float* const* exp_avgs_host, float* const* exp_avg_sqs_host, const int64_t* n_host,
+                       int* const* steps_host, double lr, double beta1, double beta2, double eps, ds_stream_t stream);
+
 /* replaces VectorAdam.step (python/diffsoup/optimize.py:36-68) for one
  * parameter of `rows` vectors of `dim` components (vertex positions: dim 3):
  * with t = *step + 1, per row

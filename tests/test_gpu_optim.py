@@ -111,3 +111,25 @@ def test_training_loop_in_one_graph_reduces_the_loss():
         losses.append(float(step.loss.item()))
     assert all(np.isfinite(losses))
     assert np.mean(losses[-10:]) < 0.9 * np.mean(losses[:5]), (losses[:5], losses[-10:])
+
+
+@pytest.mark.parametrize("sizes", [[1], [3, 2048, 2049, 4096, 7], [100000] + [5] * 40])
+def test_group_update_equals_single_updates(sizes):
+    """Parameters of a group in one launch: block edges, odd sizes, an unaligned parameter, more than one launch."""
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    mk = lambda n: torch.randn(n + 1, generator=g, device="cuda")[1:]  # noqa: E731  (not 16-byte aligned)
+    base = [torch.randn(n, generator=g, device="cuda") if i % 2 == 0 else mk(n) for i, n in enumerate(sizes)]
+    a = [t.clone() if i % 2 == 0 else t.detach() for i, t in enumerate(base)]
+    b = [t.clone().requires_grad_(True) for t in base]
+    for t in a:
+        t.requires_grad_(True)
+    oa, ob = Adam(a, lr=1e-2), torch.optim.Adam(b, lr=1e-2)
+    for _ in range(3):
+        for x, y in zip(a, b):
+            x.grad = 1e-2 * torch.randn(x.shape, generator=g, device="cuda")
+            y.grad = x.grad.clone()
+        oa.step()
+        ob.step()
+    for x, y in zip(a, b):
+        assert int(oa.state[x]["step"].item()) == 3
+        torch.testing.assert_close(x.detach(), y.detach(), rtol=0, atol=1e-6)
