@@ -48,8 +48,8 @@ METRIC = "fwd+bwd views/s @15K tris 800²: batched BF16 vs plain FP32 on one B20
 # kernels one training step launches (the ncu launch list of the bench shows them): level
 # accumulation + sigmoid (opacity and features in one), project | bin_setup, 3 scan kernels, bin_fill,
 # sort_lists | raster | shade | aux from records, aux of re-enumerated blocks | edge | accumulation
-# adjoint, project backward, finish
-KERNELS_PER_STEP = 16
+# adjoint, project backward (which closes the step)
+KERNELS_PER_STEP = 15
 # kernels one inference frame launches: project | bin_setup, 3 scan kernels, bin_fill, sort_lists |
 # raster | deferred shade
 RENDER_KERNELS_PER_FRAME = 9

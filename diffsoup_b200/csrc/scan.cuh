@@ -56,8 +56,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const In*
     if (threadIdx.x == 0) partials[blockIdx.x] = tot;
 }
 
-// Exclusive scan of nb block sums in place; partials[nb] receives the total.
-static __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(int64_t* __restrict__ partials, int64_t nb) {
+// Exclusive scan of nb block sums in place; partials[nb] (and *total, when not
+// null) receives the total.
+static __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(int64_t* __restrict__ partials, int64_t nb,
+                                                                            int64_t* __restrict__ total) {
     int64_t carry = 0;
     for (int64_t start = 0; start < nb; start += kScanThreads) {
         const int64_t i = start + threadIdx.x;
@@ -67,7 +69,10 @@ static __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(int6
         if (i < nb) partials[i] = carry + excl;
         carry += tot;
     }
-    if (threadIdx.x == 0) partials[nb] = carry;
+    if (threadIdx.x == 0) {
+        partials[nb] = carry;
+        if (total) *total = carry;
+    }
 }
 
 template <typename In, typename Out>
@@ -94,19 +99,21 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const In* __re
 }
 
 // out[i] = sum of in[0..i] (inclusive) or in[0..i) (exclusive); the total is
-// left at ((int64_t*)ws)[num_blocks] on the device.
+// left at ((int64_t*)ws)[num_blocks] on the device, and in *total_copy (device)
+// when given.
 template <typename In, typename Out>
 int device_scan(const In* in, int64_t n, Out* out, bool inclusive, void* ws, cudaStream_t st,
-                int64_t** total_dev = nullptr) {
+                int64_t** total_dev = nullptr, int64_t* total_copy = nullptr) {
     int64_t* partials = reinterpret_cast<int64_t*>(ws);
     const int64_t nb = scan_num_blocks(n);
     if (total_dev) *total_dev = partials + nb;
     if (n == 0) {
         DS_CUDA(cudaMemsetAsync(partials, 0, sizeof(int64_t), st));
+        if (total_copy) DS_CUDA(cudaMemsetAsync(total_copy, 0, sizeof(int64_t), st));
         return DS_OK;
     }
     scan_block_sums_kernel<In><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, partials);
-    scan_partials_kernel<<<1, kScanThreads, 0, st>>>(partials, nb);
+    scan_partials_kernel<<<1, kScanThreads, 0, st>>>(partials, nb, total_copy);
     scan_apply_kernel<In, Out><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, partials, out, inclusive);
     return check_launch("device_scan");
 }
@@ -120,12 +127,9 @@ constexpr int kScanOneThreads = 1024;
 constexpr int kScanOneItems = 4;
 constexpr int64_t kScanOneMax = (int64_t)kScanOneThreads * kScanOneItems;
 
-// out[i] = sum of in[0..i) for i < n and out[n] = the total (n <= kScanOneMax);
-// zero[0..n) is cleared on the way (a per-item cursor of the next pass; may
-// be null).
+// out[i] = sum of in[0..i) for i < n and out[n] = the total (n <= kScanOneMax).
 static __global__ void __launch_bounds__(kScanOneThreads) scan_one_cta_kernel(const int* __restrict__ in, int n,
-                                                                              int64_t* __restrict__ out,
-                                                                              int* __restrict__ zero) {
+                                                                              int64_t* __restrict__ out) {
     __shared__ int64_t warp_tot[kScanOneThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = (n + kScanOneThreads - 1) / kScanOneThreads;  // <= kScanOneItems
@@ -151,7 +155,6 @@ static __global__ void __launch_bounds__(kScanOneThreads) scan_one_cta_kernel(co
     for (int i = i0; i < i1; ++i) {
         out[i] = run;
         run += in[i];
-        if (zero) zero[i] = 0;
     }
     if (threadIdx.x == 0) out[n] = total;
 }

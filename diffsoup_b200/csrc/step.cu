@@ -399,21 +399,34 @@ __global__ void __launch_bounds__(kThreads) project_kernel(int B, int V, const f
     reinterpret_cast<float4*>(pos)[i] = o;
 }
 
-// grad_verts[v] = sum_b mvp[b][:, :3]^T grad_pos[b][v]
+// grad_verts[v] = sum_b mvp[b][:, :3]^T grad_pos[b][v]; the first thread also
+// closes the step: the loss, the next iteration of the opacity-threshold RNG
+// and the status of re-enumerated blocks.
 __global__ void __launch_bounds__(kThreads) project_backward_kernel(int B, int V, const float* __restrict__ mvp,
                                                                     const double* __restrict__ grad_pos,
-                                                                    float* __restrict__ grad_verts) {
+                                                                    float* __restrict__ grad_verts,
+                                                                    const double* __restrict__ loss_sum, float inv_n,
+                                                                    float* __restrict__ loss, uint64_t* __restrict__ rng,
+                                                                    const int* __restrict__ rec_counters,
+                                                                    int* __restrict__ status) {
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        *loss = (float)(*loss_sum * (double)inv_n);
+        if (rng) rng[1] += 1;
+        if (status && rec_counters[1] > 0) atomicOr(status, DS_STATUS_RECORD_FALLBACK);
+    }
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     double gx = 0.0, gy = 0.0, gz = 0.0;
     for (int b = 0; b < B; ++b) {
         const float* M = mvp + (size_t)b * 16;
-        const double* gp = grad_pos + ((size_t)b * V + v) * 4;
+        const double2* gp = reinterpret_cast<const double2*>(grad_pos + ((size_t)b * V + v) * 4);
+        const double2 g01 = gp[0], g23 = gp[1];
+        const double g[4] = {g01.x, g01.y, g23.x, g23.y};
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            gx += (double)M[r * 4 + 0] * gp[r];
-            gy += (double)M[r * 4 + 1] * gp[r];
-            gz += (double)M[r * 4 + 2] * gp[r];
+            gx += (double)M[r * 4 + 0] * g[r];
+            gy += (double)M[r * 4 + 1] * g[r];
+            gz += (double)M[r * 4 + 2] * g[r];
         }
     }
     grad_verts[(size_t)v * 3] = (float)gx;
@@ -539,16 +552,6 @@ __global__ void __launch_bounds__(kEdgeThreads, DSB_EDGE_MIN_CTAS) edge_step_ker
             for (int j = 0; j < 4; ++j)
                 if (acc.g[k * 4 + j] != 0.f) atomicAdd(gp + (size_t)v * 4 + j, (double)acc.g[k * 4 + j]);
         }
-    }
-}
-
-__global__ void finish_kernel(const double* __restrict__ loss_sum, float inv_n, float* __restrict__ loss,
-                              uint64_t* __restrict__ rng, const int* __restrict__ rec_counters,
-                              int* __restrict__ status) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        *loss = (float)(*loss_sum * (double)inv_n);
-        if (rng) rng[1] += 1;  // next iteration of the opacity-threshold RNG
-        if (status && rec_counters[1] > 0) atomicOr(status, DS_STATUS_RECORD_FALLBACK);
     }
 }
 
@@ -865,16 +868,16 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
 
     int rc = mark(0, st);
     if (rc) return rc;
-    // zero the accumulators of this step
-    DS_CUDA(cudaMemsetAsync(w.grad_pos, 0,
-                            reinterpret_cast<char*>(w.rec_counters + 2) - reinterpret_cast<char*>(w.grad_pos), st));
-    DS_CUDA(cudaMemsetAsync(grad_mlp_params, 0, sizeof(float) * ds_step_mlp_param_count(&c), st));
-
     // Side stream for independent parts; the phase events (profiling) time
     // the phases one after another on st instead.
     SideStream* side = g_step_nevents == 0 ? side_stream() : nullptr;
     const cudaStream_t sst = side ? side->s : st;
     if (side && (rc = fork_to(side, 0, st))) return rc;
+
+    // zero the accumulators of this step, beside the level accumulation
+    DS_CUDA(cudaMemsetAsync(w.grad_pos, 0,
+                            reinterpret_cast<char*>(w.rec_counters + 2) - reinterpret_cast<char*>(w.grad_pos), st));
+    DS_CUDA(cudaMemsetAsync(grad_mlp_params, 0, sizeof(float) * ds_step_mlp_param_count(&c), st));
 
     // prep: opacity and feature accumulation + sigmoid (side), projection (st)
     const unsigned tb = (unsigned)((c.T + kPrepWarps - 1) / kPrepWarps);
@@ -983,8 +986,9 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
     // (one stream: the phases in order, so that the profiling events time each alone)
     if (!side && (rc = accum_backward(st))) return rc;
     // adjoint of the projection
-    if (c.V > 0) project_backward_kernel<<<blocks_for(c.V), kThreads, 0, st>>>(c.B, c.V, mvp, w.grad_pos, grad_verts);
-    finish_kernel<<<1, 32, 0, st>>>(w.loss_sum, a.inv_n, loss, c.stochastic ? rng : nullptr, w.rec_counters, status);
+    project_backward_kernel<<<blocks_for(c.V > 0 ? c.V : 1), kThreads, 0, st>>>(
+        c.B, c.V, mvp, w.grad_pos, grad_verts, w.loss_sum, a.inv_n, loss, c.stochastic ? rng : nullptr,
+        w.rec_counters, status);
     if ((rc = mark(7, st))) return rc;
     return check_launch("train_step");
 }

@@ -51,7 +51,7 @@ struct TileWs {
     int* sorted;       // per tile: 1 when its list is ordered by zlo
     ListEntry* list;
     ListEntry* fill;   // the fill pass's unsorted lists (same offsets)
-    int* work;         // persistent-kernel work counters [2]
+    int* work;         // persistent-kernel work counters [2], then the status word of ds_tiles_bin_report
     void* scan;
 };
 
@@ -511,9 +511,15 @@ __device__ __forceinline__ bool box_overlaps(const TriBox& r, const BlockGeom& g
     return r.y0 < g.wy0 + g.bh && r.y1 > g.wy0 && r.x0 < g.wx0 + g.bw && r.x1 > g.wx0;
 }
 
-__device__ __forceinline__ int warp_next(int* work) {
+// The warp's next item of `items`.  Every warp of the grid ends on one value at or
+// past `items`, so the warp that draws the last of them puts the counter back to
+// zero for the next kernel (the binning pass cleared it first).
+__device__ __forceinline__ int warp_next(int* work, int items) {
     int item = 0;
-    if ((threadIdx.x & 31) == 0) item = atomicAdd(work, 1);
+    if ((threadIdx.x & 31) == 0) {
+        item = atomicAdd(work, 1);
+        if (item == items + (int)(gridDim.x * (blockDim.x >> 5)) - 1) *work = 0;
+    }
     return __shfl_sync(0xffffffffu, item, 0);
 }
 
@@ -692,7 +698,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
     if (thr_mode == 1) { seed = rng[0]; iter = (uint32_t)rng[1]; }
     int cid = -1, cfill = 0;  // REC: the warp's current record chunk
     const int items = num_tiles * kBlocksPerTile;
-    for (int item = warp_next(work); item < items; item = warp_next(work)) {
+    for (int item = warp_next(work, items); item < items; item = warp_next(work, items)) {
         const BlockGeom g = block_geometry(item, B, views, T, offsets, sorted, capacity, bwl);
         if (g.begin >= g.end) {  // no candidate: background (a quarter to a third of the blocks)
             if (g.valid) reinterpret_cast<float4*>(rast)[g.pix] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -886,7 +892,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
         for (int k = lane; k < S; k += 32) s_acc[warp][k] = 0.f;
     __syncwarp();
     const int items = item_list ? *item_count : num_tiles * kBlocksPerTile;
-    for (int n = warp_next(work); n < items; n = warp_next(work)) {
+    for (int n = warp_next(work, items); n < items; n = warp_next(work, items)) {
         const int item = item_list ? item_list[n] : n;
         const BlockGeom g = block_geometry(item, B, views, T, offsets, sorted, capacity, bwl);
         const float ndc_x = pix_ndc(g.px, g.W), ndc_y = pix_ndc(g.py, g.H);
@@ -988,10 +994,9 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     TileWs w = carve(workspace, B, T, num_tiles, list_capacity, nullptr);
-    // up to kScanOneMax tiles, one launch scans the counts, writes the total and clears the fill cursors
-    const bool one_cta = num_tiles <= kScanOneMax;
-    DS_CUDA(cudaMemsetAsync(w.counts, 0, (size_t)num_tiles * sizeof(int), st));
-    if (!one_cta) DS_CUDA(cudaMemsetAsync(w.cursor, 0, (size_t)num_tiles * sizeof(int), st));
+    // one memset clears the counts, the fill cursors, the work counters and the workspace's status word
+    // (counts .. work; the offsets and flags in between are written below): a launch costs more than their bytes
+    DS_CUDA(cudaMemsetAsync(w.counts, 0, reinterpret_cast<char*>(w.work + 3) - reinterpret_cast<char*>(w.counts), st));
     const int64_t n = (int64_t)B * T;
     const bool narrow = n <= kBinNarrow;
     const unsigned grid = blocks_for(narrow ? n * 4 : n);  // 8 or 32 triangles per warp
@@ -999,14 +1004,13 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
         const auto setup = narrow ? bin_setup_kernel<8> : bin_setup_kernel<32>;
         setup<<<grid, kThreads, 0, st>>>(B, views, V, pos, T, tri, w.boxes, w.verts, w.ndc, w.edges, w.counts);
     }
-    if (one_cta) {
-        scan_one_cta_kernel<<<1, kScanOneThreads, 0, st>>>(w.counts, num_tiles, w.offsets, w.cursor);
+    // offsets[num_tiles] = total number of entries; up to kScanOneMax tiles in one launch
+    if (num_tiles <= kScanOneMax) {
+        scan_one_cta_kernel<<<1, kScanOneThreads, 0, st>>>(w.counts, num_tiles, w.offsets);
     } else {
-        int64_t* total_dev = nullptr;
-        rc = device_scan<int, int64_t>(w.counts, num_tiles, w.offsets, false, w.scan, st, &total_dev);
+        rc = device_scan<int, int64_t>(w.counts, num_tiles, w.offsets, false, w.scan, st, nullptr,
+                                       w.offsets + num_tiles);
         if (rc) return rc;
-        // offsets[num_tiles] = total number of entries
-        DS_CUDA(cudaMemcpyAsync(w.offsets + num_tiles, total_dev, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
     }
     if (n > 0) {
         const auto fill = narrow ? bin_fill_kernel<8> : bin_fill_kernel<32>;
@@ -1017,6 +1021,24 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
         sort_lists_kernel<<<(unsigned)((num_tiles + kSortWarps - 1) / kSortWarps), kSortWarps * 32, 0, st>>>(
             num_tiles, w.offsets, w.fill, w.list, list_capacity, w.sorted);
     return check_launch("tiles_bin");
+}
+
+size_t ds_tiles_status_offset(int B, int T, int num_tiles, int64_t list_capacity) {
+    const TileWs w = carve(nullptr, B, T, num_tiles, list_capacity, nullptr);
+    return (size_t)(reinterpret_cast<const char*>(w.work + 2) - (const char*)nullptr);
+}
+
+int ds_tiles_bin_report(int B, const ds_view_desc* views, int num_tiles, int V, const float* pos, int T, const int* tri,
+                        void* workspace, size_t workspace_bytes, int64_t list_capacity, int* status_host,
+                        ds_stream_t stream) {
+    const int rc0 = check_tiles_args(B, views, num_tiles, V, pos, T, workspace_bytes, list_capacity);
+    if (rc0) return rc0;
+    int* status = carve(workspace, B, T, num_tiles, list_capacity, nullptr).work + 2;
+    const int rc = ds_tiles_bin(B, views, num_tiles, V, pos, T, tri, workspace, workspace_bytes, list_capacity, status,
+                                stream);
+    if (rc) return rc;
+    DS_CUDA(cudaMemcpyAsync(status_host, status, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    return DS_OK;
 }
 
 }  // extern "C"
@@ -1046,7 +1068,6 @@ int tiles_rasterize_impl(int B, const ds_view_desc* views, int num_tiles, int T,
                          void* workspace, int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl) {
     if (num_tiles == 0) return DS_OK;
     TileWs w = carve(workspace, B, T, num_tiles, list_capacity, nullptr);
-    DS_CUDA(cudaMemsetAsync(w.work, 0, sizeof(int), st));
     if (rs != nullptr) {
         const void* k = reinterpret_cast<const void*>(&raster_kernel<true>);
         raster_kernel<true><<<block_grid(num_tiles, k, g_occ_raster_rec), kWarpsPerCta * 32, 0, st>>>(
@@ -1066,7 +1087,6 @@ static int aux_launch(int B, const ds_view_desc* views, int num_tiles, int T, in
                       float scale, float* grad_alpha_src, void* workspace, int64_t list_capacity,
                       const int* item_list, const int* item_count, cudaStream_t st, int bwl) {
     TileWs w = carve(workspace, B, T, num_tiles, list_capacity, nullptr);
-    DS_CUDA(cudaMemsetAsync(w.work + 1, 0, sizeof(int), st));
     const void* k = reinterpret_cast<const void*>(&aux_kernel);
     aux_kernel<<<block_grid(num_tiles, k, g_occ_aux), kWarpsPerCta * 32, 0, st>>>(
         B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,

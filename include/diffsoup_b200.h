@@ -198,6 +198,14 @@ size_t ds_tiles_workspace_size(int B, int T, int num_tiles, int64_t list_capacit
 int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const float* pos, int T, const int* tri,
                  void* workspace, size_t workspace_bytes, int64_t list_capacity, int* status, ds_stream_t stream);
 
+/* ds_tiles_bin with the status word inside the workspace (cleared with the
+ * bins, at ds_tiles_status_offset bytes) and an asynchronous copy of it to
+ * *status_host (page-locked host memory that outlives the copy). */
+size_t ds_tiles_status_offset(int B, int T, int num_tiles, int64_t list_capacity);
+int ds_tiles_bin_report(int B, const ds_view_desc* views, int num_tiles, int V, const float* pos, int T, const int* tri,
+                        void* workspace, size_t workspace_bytes, int64_t list_capacity, int* status_host,
+                        ds_stream_t stream);
+
 /* Tiled forward rasterizer with stochastic opacity (replaces
  * rasterize_multires_triangle_alpha, python/diffsoup/multires.py:52-102:
  * multires_triangle_alpha + threshold + depth_test).  Uses the bins of the
