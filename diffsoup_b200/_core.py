@@ -74,6 +74,8 @@ _sig("ds_make_view_table", _i32, _i32, C.POINTER(C.c_int), C.POINTER(C.c_int), C
      C.POINTER(C.c_int64))
 _sig("ds_tiles_workspace_size", _sz, _i32, _i32, _i32, _i64)
 _sig("ds_tiles_bin", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _vp, _sz, _i64, _vp, _vp)
+_sig("ds_tiles_status_offset", _sz, _i32, _i32, _i32, _i64)
+_sig("ds_tiles_bin_report", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _vp, _sz, _i64, _vp, _vp)
 _sig("ds_tiles_rasterize", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _i32, _i32, _vp, _i32, _f32, _vp, _vp, _vp,
      _sz, _i64, _vp)
 _sig("ds_tiles_opacity_aux", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _vp, _vp, _f32,
@@ -108,7 +110,8 @@ def ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
 
 
 def stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the raw handle: a torch.cuda.Stream object costs 3 us per call
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _cuda_contig(name: str, t: torch.Tensor, dtype: torch.dtype, ndim: int) -> None:

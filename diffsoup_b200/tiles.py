@@ -14,6 +14,7 @@ host synchronisation is needed.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -26,7 +27,8 @@ DS_STATUS_LIST_OVERFLOW = 1
 DS_STATUS_RECORD_FALLBACK = 2
 
 _capacity: Dict[int, int] = {}
-_pending_status: Dict[int, Tuple[torch.Tensor, torch.cuda.Event, int]] = {}
+# per device: (status slot, capacity) of the last binning whose status has not been looked at
+_pending_status: Dict[int, Tuple[int, int]] = {}
 _view_tables: Dict[Tuple, Tuple[torch.Tensor, int, int, List[int]]] = {}
 
 
@@ -53,6 +55,30 @@ def view_table(hw: Sequence[Tuple[int, int]], device: torch.device):
     return out
 
 
+# Status words of the last binning calls in page-locked memory.  A call takes the
+# next slot, puts -1 there, and the device copies its status (>= 0) over it, so a
+# slot is read without an event or a synchronisation.  A late copy into a slot
+# taken again only shows an older call's status.
+_SLOTS = 256
+_slots: List = []  # [tensor, ctypes view], once allocated
+_next_slot = itertools.count()
+
+
+def _status_slots():
+    if not _slots:
+        t = torch.full((_SLOTS,), -1, dtype=torch.int32, pin_memory=True)
+        _slots[:] = [t, (C.c_int32 * _SLOTS).from_address(t.data_ptr())]
+    return _slots
+
+
+def copy_status(status: torch.Tensor):
+    """Queues a copy of a status word (int32 [1], device) to the host; the returned
+    function reads it once the stream has been synchronised."""
+    slots, slot = _status_slots(), next(_next_slot) % _SLOTS
+    slots[0][slot:slot + 1].copy_(status, non_blocking=True)
+    return lambda: int(slots[1][slot])
+
+
 def _device_index(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
@@ -61,11 +87,12 @@ def _capacity_for(device: torch.device, B: int, T: int) -> int:
     di = _device_index(device)
     pend = _pending_status.get(di)
     if pend is not None:
-        status, ev, cap = pend
-        if ev.query():
-            if int(status.item()) & DS_STATUS_LIST_OVERFLOW:
+        slot, cap = pend
+        status = _status_slots()[1][slot]
+        if status >= 0:
+            if status & DS_STATUS_LIST_OVERFLOW:
                 _capacity[di] = max(_capacity.get(di, 0), 2 * cap)
-            del _pending_status[di]
+            _pending_status.pop(di, None)
     want = max(1 << 16, 8 * B * T)
     cap = max(_capacity.get(di, 0), want)
     _capacity[di] = cap
@@ -84,10 +111,15 @@ class Bins:
     pix_offsets: List[int]
     capacity: int
     workspace: torch.Tensor
-    status: torch.Tensor
     pos: torch.Tensor
     tri: torch.Tensor
     key: Tuple
+
+    @property
+    def status(self) -> torch.Tensor:
+        """The status word (int32 [1], device) of the binning call."""
+        o = int(_core.lib.ds_tiles_status_offset(self.B, self.T, self.num_tiles, self.capacity))
+        return self.workspace[o:o + 4].view(torch.int32)
 
 
 _last: Optional[Bins] = None
@@ -95,7 +127,7 @@ _last: Optional[Bins] = None
 
 def _key(pos: torch.Tensor, tri: torch.Tensor, hw) -> Tuple:
     return (pos.data_ptr(), pos._version, tuple(pos.shape), tri.data_ptr(), tri._version, tuple(tri.shape),
-            tuple(hw), torch.cuda.current_stream(pos.device).cuda_stream)
+            hw, torch._C._cuda_getCurrentRawStream(_device_index(pos.device)))
 
 
 def bin_views(pos: torch.Tensor, tri: torch.Tensor, hw: Sequence[Tuple[int, int]], reuse: bool = True) -> Bins:
@@ -111,15 +143,13 @@ def bin_views(pos: torch.Tensor, tri: torch.Tensor, hw: Sequence[Tuple[int, int]
     table, nt, npix, offs = view_table(hw, dev)
     cap = _capacity_for(dev, B, T)
     ws = _core.workspace(_core.lib.ds_tiles_workspace_size(B, T, nt, cap), dev)
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
-    _core.check(_core.lib.ds_tiles_bin(B, _core.ptr(table), nt, V, _core.ptr(pos), T, _core.ptr(tri), _core.ptr(ws),
-                                       ws.numel(), cap, _core.ptr(status), _core.stream()))
-    host = torch.empty(1, dtype=torch.int32, pin_memory=True)
-    host.copy_(status, non_blocking=True)
-    ev = torch.cuda.Event()
-    ev.record()
-    _pending_status[_device_index(dev)] = (host, ev, cap)
-    bins = Bins(B, T, V, hw, table, nt, npix, offs, cap, ws, status, pos, tri, key)
+    slots, slot = _status_slots(), next(_next_slot) % _SLOTS
+    slots[1][slot] = -1
+    _core.check(_core.lib.ds_tiles_bin_report(B, _core.ptr(table), nt, V, _core.ptr(pos), T, _core.ptr(tri),
+                                              _core.ptr(ws), ws.numel(), cap, slots[0].data_ptr() + 4 * slot,
+                                              _core.stream()))
+    _pending_status[_device_index(dev)] = (slot, cap)
+    bins = Bins(B, T, V, hw, table, nt, npix, offs, cap, ws, pos, tri, key)
     _last = bins
     return bins
 

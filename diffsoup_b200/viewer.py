@@ -163,17 +163,20 @@ class Renderer:
         (as a tuple in that order)."""
         m = torch.as_tensor(mvps, dtype=torch.float32).reshape(-1, 4, 4)
         f = self._frame(m.shape[0], int(height), int(width))
-        f.set_views(m)
+        # everything up to the one synchronisation is queued without waiting: the views' copy, the frame, the
+        # results' copies and the status word
+        f.set_views(m, wait=False)
         f.status.zero_()
         f.run(want_rgb=rgb)
-        torch.cuda.current_stream(self.device).synchronize()
-        if f.overflowed():
-            f.grow()  # this frame is exact all the same; the next ones bin without overflow
         out = [f.rgba8.view(f.B, f.H, f.W, 4).clone()]
         if rgb:
             out.append(f.rgb.view(f.B, f.H, f.W, 3).clone())
         if gbuf:
             out.append(f.gbuf.view(f.B, f.H, f.W, 4).clone())
+        status = _tiles.copy_status(f.status)
+        torch.cuda.current_stream(self.device).synchronize()
+        if status() & _tiles.DS_STATUS_LIST_OVERFLOW:
+            f.grow()  # this frame is exact all the same; the next ones bin without overflow
         return out[0] if len(out) == 1 else tuple(out)
 
     def frame(self, mvps, height: int, width: int) -> "_Frame":
@@ -202,8 +205,8 @@ class _Frame:
         dev = r.device
         with torch.cuda.device(dev):
             self.views, self.num_tiles, self.num_pixels, _ = _tiles.view_table([(H, W)] * B, dev)
-            self.mvp = torch.zeros(B, 16, dtype=torch.float32, device=dev)
-            self.inv_mvp = torch.zeros(B, 16, dtype=torch.float32, device=dev)
+            self.matrices = torch.zeros(2, B, 16, dtype=torch.float32, device=dev)  # MVPs and their inverses
+            self.mvp, self.inv_mvp = self.matrices[0], self.matrices[1]
             self.gbuf = torch.empty(self.num_pixels, 4, dtype=torch.float32, device=dev)
             self.rgb = torch.empty(self.num_pixels, 3, dtype=torch.float32, device=dev)
             self.rgba8 = torch.empty(self.num_pixels, 4, dtype=torch.uint8, device=dev)
@@ -239,13 +242,14 @@ class _Frame:
             self.grow()
         raise RuntimeError("render: bin-list capacity did not converge")
 
-    def set_views(self, mvps: torch.Tensor) -> None:
+    def set_views(self, mvps: torch.Tensor, wait: bool = True) -> None:
         """Row-major MVPs [B,4,4] and their inverses (FP64 on the host, then
-        FP32, as glm::inverse gives the viewer's uInvMVP)."""
+        FP32, as glm::inverse gives the viewer's uInvMVP), in one copy.  Without
+        `wait` only work on the current stream sees them (the host buffer is staged
+        by the time this returns)."""
         m = mvps.detach().to("cpu", torch.float64).reshape(self.B, 4, 4)
-        inv = torch.linalg.inv(m)
-        self.mvp.copy_(m.reshape(self.B, 16).float(), non_blocking=False)
-        self.inv_mvp.copy_(inv.reshape(self.B, 16).float(), non_blocking=False)
+        both = torch.stack((m, torch.linalg.inv(m))).reshape(2, self.B, 16).float()
+        self.matrices.copy_(both, non_blocking=not wait)
 
     def run(self, want_rgb: bool = False) -> None:
         r = self.r
