@@ -74,6 +74,9 @@ _sig("ds_make_view_table", _i32, _i32, C.POINTER(C.c_int), C.POINTER(C.c_int), C
      C.POINTER(C.c_int64))
 _sig("ds_tiles_workspace_size", _sz, _i32, _i32, _i32, _i64)
 _sig("ds_tiles_bin", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _vp, _sz, _i64, _vp, _vp)
+_sig("ds_color_mlp_forward", _i32, _i64, _i32, _i32, _i32, *([_vp] * 8))
+_sig("ds_color_mlp_backward_workspace", _sz, _i64, _i32, _i32)
+_sig("ds_color_mlp_backward", _i32, _i64, _i32, _i32, _i32, *([_vp] * 13), _sz, _vp)
 _sig("ds_tiles_status_offset", _sz, _i32, _i32, _i32, _i64)
 _sig("ds_tiles_bin_report", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _vp, _sz, _i64, _vp, _vp)
 _sig("ds_tiles_rasterize", _i32, _i32, _vp, _i32, _i32, _vp, _i32, _vp, _i32, _i32, _vp, _i32, _f32, _vp, _vp, _vp,

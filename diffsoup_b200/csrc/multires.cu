@@ -5,6 +5,7 @@
 // the scatters use vector atomics (red.global.add.v4.f32, sm_90+) so one
 // instruction updates four channels.
 #include "lattice_map.cuh"
+#include "rows.cuh"
 
 namespace dsb {
 
@@ -121,26 +122,6 @@ struct Row7 {
         atomicAdd(p + one, o * w);
     }
 };
-
-// Warp-wide copy between 32 rows of K floats, lane's row at tile + lane * K, and
-// `live` consecutive rows at g (16-byte aligned when all 32 are live).
-template <bool STORE>
-__device__ __forceinline__ void warp_rows(float* tile, float* g, int K, int live) {
-    const int lane = threadIdx.x & 31;
-    if (!STORE) __syncwarp();
-    if (live == 32 && ((uintptr_t)g & 15) == 0) {
-        for (int i = lane; i < 8 * K; i += 32) {
-            float4* t = reinterpret_cast<float4*>(tile) + i;
-            float4* o = reinterpret_cast<float4*>(g) + i;
-            if (STORE) *o = *t; else *t = __ldg(o);
-        }
-    } else {
-        for (int i = lane; i < live * K; i += 32) {
-            if (STORE) g[i] = tile[i]; else tile[i] = __ldg(g + i);
-        }
-    }
-    __syncwarp();
-}
 
 // color_kernel with every pixel written (background pixels zero): no zeroed
 // buffer and no read of it.  Channel counts that are no multiple of four go

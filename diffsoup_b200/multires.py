@@ -82,6 +82,71 @@ def rasterize_multires_triangle_alpha(resolution: Tuple[int, int], pos: torch.Te
 #  Colour MLP (multires.py:109-207)
 # ---------------------------------------------------------------------------
 
+def _shade(x: torch.Tensor, mask: Optional[torch.Tensor], weights, biases: torch.Tensor) -> torch.Tensor:
+    """The fused kernels' function of flat rows x [n,in], in torch operations (their double backward)."""
+    h, o = x, 0
+    for w in weights:
+        h = nn.functional.linear(h, w, biases[o:o + w.shape[0]])
+        o += w.shape[0]
+        h = torch.sigmoid(h) if w is weights[-1] else torch.relu(h)
+    y = (1.0 - x[:, 3:4]) * x[:, :3] + x[:, 3:4] * h
+    return y if mask is None else torch.where(mask.unsqueeze(-1), y, torch.zeros_like(y))
+
+
+class _ColorMLPFn(torch.autograd.Function):
+    """ColorMLP on flat rows by ds_color_mlp_forward / _backward (csrc/color_mlp.cu)."""
+
+    @staticmethod
+    def forward(ctx, x, mask, biases, *weights):
+        n, cin = x.shape
+        out = torch.empty(n, 3, dtype=torch.float32, device=x.device)
+        p = _core.ptr
+        w1 = weights[1] if len(weights) == 3 else None
+        _core.check(_core.lib.ds_color_mlp_forward(n, cin, 16, len(weights) - 1, p(x), p(mask), p(weights[0]), p(w1),
+                                                   p(weights[-1]), p(biases), p(out), _core.stream()))
+        ctx.save_for_backward(x, mask, biases, *weights)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        x, mask, biases, *weights = ctx.saved_tensors
+        if torch.is_grad_enabled():  # create_graph: the gradient as differentiable operations
+            ins = [t for t, need in zip((x, biases, *weights), (ctx.needs_input_grad[0], *ctx.needs_input_grad[2:]))
+                   if need]
+            grads = iter(torch.autograd.grad(_shade(x, mask, weights, biases), ins, grad_out, create_graph=True))
+            need = ctx.needs_input_grad
+            return (next(grads) if need[0] else None, None, *(next(grads) if k else None for k in need[2:]))
+        n, cin = x.shape
+        layers = len(weights) - 1
+        grad_out = grad_out.contiguous()
+        gx = torch.empty_like(x) if ctx.needs_input_grad[0] else None
+        gb = torch.empty_like(biases)
+        gw = [torch.empty_like(w) for w in weights]
+        ws = _core.workspace(_core.lib.ds_color_mlp_backward_workspace(n, cin, layers), x.device)
+        p, two = _core.ptr, len(weights) == 3
+        _core.check(_core.lib.ds_color_mlp_backward(
+            n, cin, 16, layers, p(x), p(mask), p(weights[0]), p(weights[1] if two else None), p(weights[-1]), p(biases),
+            p(grad_out), p(gx), p(gw[0]), p(gw[1] if two else None), p(gw[-1]), p(gb), p(ws), ws.numel(),
+            _core.stream()))
+        return (gx, None, gb, *gw)
+
+
+def _plain_call(*tensors) -> bool:
+    """Whether nothing watches or transforms torch operations on these tensors (tracing, compilation, function
+    transforms, forward-mode AD, dispatch modes, autocast), so that a kernel may take their place."""
+    return (all(type(t) in (torch.Tensor, nn.Parameter) for t in tensors)
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and not torch.is_autocast_enabled("cuda")
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
+
+
+def _no_hooks(module: nn.Module) -> bool:
+    return not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                or module._backward_pre_hooks or "forward" in module.__dict__)
+
+
 class ColorMLP(nn.Module):
     """Per-pixel shading MLP with a residual blend.
 
@@ -117,10 +182,48 @@ class ColorMLP(nn.Module):
             nn.init.xavier_uniform_(last.weight, gain=1.0)
         nn.init.zeros_(last.bias)
 
+    def _fused_layers(self, x: torch.Tensor, mask: Optional[torch.Tensor]):
+        """The Linear layers when the fused kernels compute exactly this call: FP32 on the current CUDA device,
+        4 to 20 inputs, one or two hidden layers of 16, three outputs, and the plain module as built here."""
+        mods = list(self.mlp) if type(self.mlp) is nn.Sequential else []
+        kinds = [type(m) for m in mods]
+        if kinds not in ([nn.Linear, nn.ReLU] * n + [nn.Linear, nn.Sigmoid] for n in (1, 2)):
+            return None
+        lins = mods[0::2]
+        shapes = [(16, self.input_dim)] + [(16, 16)] * (len(lins) - 2) + [(3, 16)]
+        g = nn.modules.module
+        if (not 4 <= self.input_dim <= 20 or self.output_dim != 3 or x.numel() == 0
+                or not (x.is_cuda and x.dtype == torch.float32 and x.device.index == torch.cuda.current_device())
+                or (mask is not None and not (type(mask) is torch.Tensor and mask.dtype == torch.bool
+                                              and mask.device == x.device))
+                or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+                or g._global_backward_pre_hooks or not all(_no_hooks(m) for m in mods + [self.mlp])):
+            return None
+        for lin, shape in zip(lins, shapes):
+            if lin.bias is None or tuple(lin.weight.shape) != shape or any(
+                    t.device != x.device or t.dtype != torch.float32 or not t.is_contiguous()
+                    for t in (lin.weight, lin.bias)):
+                return None
+        return lins if _plain_call(x, *(t for lin in lins for t in (lin.weight, lin.bias))) else None
+
     def forward(self, x: torch.Tensor, mask: Optional[torch.Tensor] = None) -> torch.Tensor:
         B, H, W, _ = x.shape
         assert x.shape == (B, H, W, self.input_dim)
         assert mask is None or mask.shape == (B, H, W)
+        lins = self._fused_layers(x, mask)
+        if lins is not None:
+            weights = [lin.weight for lin in lins]
+            biases = torch.cat([lin.bias for lin in lins])
+            if mask is None:
+                return _ColorMLPFn.apply(x.reshape(-1, self.input_dim).contiguous(), None, biases,
+                                         *weights).view(B, H, W, 3)
+            if not mask.any():
+                return torch.zeros(B, H, W, 3, device=x.device, dtype=x.dtype)
+            rows, flags = x.reshape(-1, self.input_dim).contiguous(), mask.reshape(-1).contiguous()
+            if torch.is_grad_enabled():
+                # copies: writing to x or mask before backward is allowed here, as it is when rows are gathered
+                rows, flags = rows.clone(), flags.clone()
+            return _ColorMLPFn.apply(rows, flags, biases, *weights).view(B, H, W, 3)
         rgb, res = x[..., :3], x[..., 3:4]
         if mask is None:
             y = self.mlp(x.reshape(-1, self.input_dim)).view(B, H, W, self.output_dim)

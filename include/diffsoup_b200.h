@@ -163,6 +163,22 @@ int ds_accumulate_to_level_backward(int T, int min_level, int max_level, int tar
 int ds_accumulate_to_level_backward_set(int T, int min_level, int max_level, int target_level, int S, int S_target,
                                         int C, float* grad_features, const float* grad_out, ds_stream_t stream);
 
+/* ColorMLP.forward (python/diffsoup/multires.py:169-207) for hidden width 16,
+ * one or two hidden layers, 4 to 20 inputs and three outputs, in FP32:
+ * out [n,3] = (1 - x3) x[0:3] + x3 sigmoid(MLP(x)) where mask (bytes, NULL: all
+ * pixels), else 0.  Weights in torch.nn.Linear layout; biases = b0 [16],
+ * b1 [16] (two layers), bo [3].  w1 is NULL with one layer. */
+int ds_color_mlp_forward(int64_t n, int in, int hidden, int layers, const float* x, const unsigned char* mask,
+                         const float* w0, const float* w1, const float* wo, const float* biases, float* out,
+                         ds_stream_t stream);
+
+/* Its gradients (overwritten; grad_x [n,in] may be NULL). */
+size_t ds_color_mlp_backward_workspace(int64_t n, int in, int layers);
+int ds_color_mlp_backward(int64_t n, int in, int hidden, int layers, const float* x, const unsigned char* mask,
+                          const float* w0, const float* w1, const float* wo, const float* biases,
+                          const float* grad_out, float* grad_x, float* grad_w0, float* grad_w1, float* grad_wo,
+                          float* grad_biases, void* workspace, size_t workspace_bytes, ds_stream_t stream);
+
 /* ===================================================================== */
 /*  B200 path: screen-tile binning, tiled rasterizer, tiled aux gradient  */
 /* ===================================================================== */
