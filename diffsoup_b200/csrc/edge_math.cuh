@@ -118,6 +118,55 @@ __device__ __forceinline__ void add_mid_contrib(float mx, float my, const float4
     a.any = true;
 }
 
+// Silhouette contribution at the crossing of the pixel pair with the triangle's
+// edge (rasterize.cu:866-891).
+__device__ __forceinline__ void edge_crossing_contrib(const float4 P0[3], float nx0, float ny0, float nx1, float ny1,
+                                                      float gx, float gy, EdgeAccum& acc) {
+    int i0, i1;
+    float s0, s1;
+    if (!find_edge_intersection(P0, nx0, ny0, nx1, ny1, i0, i1, s0, s1)) return;
+    const float4 A = i0 == 0 ? P0[0] : (i0 == 1 ? P0[1] : P0[2]);
+    const float4 Bv = i1 == 0 ? P0[0] : (i1 == 1 ? P0[1] : P0[2]);
+    const float cx = s0 * A.x + s1 * Bv.x;
+    const float cy = s0 * A.y + s1 * Bv.y;
+    const float cw = s0 * A.w + s1 * Bv.w;
+    const float iw = 1.f / cw, iw2 = iw * iw;
+    const float gsum = gx * cx + gy * cy;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // static indices: no local-memory array
+        const float s = k == i0 ? s0 : (k == i1 ? s1 : 0.f);
+        if (k == i0 || k == i1) {
+            acc.g[k * 4 + 0] += s * gx * iw;
+            acc.g[k * 4 + 1] += s * gy * iw;
+            acc.g[k * 4 + 3] += -s * gsum * iw2;
+        }
+    }
+    acc.any = true;
+}
+
+// Contribution of a pair across which the neighbour's triangle P1 hides P0: a
+// triangle intersection when P1 lies behind P0 at the pixel (rasterize.cu:775-809).
+__device__ __forceinline__ void intersection_contrib(const float4 P0[3], const float4 P1[3], float depth0, float nx0,
+                                                     float ny0, float nx1, float ny1, int DX, float gx, float gy,
+                                                     EdgeAccum& acc) {
+    float tb0, tb1, cz0, cw0;
+    if (!intersect_triangle(ny0, nx0, P1[0], P1[1], P1[2], tb0, tb1, cz0, cw0)) return;
+    if (!(depth0 < cz0 / cw0)) return;
+    float nv[3], nf[3];
+    if (!(tri_normal_ndc(P0, nv) && tri_normal_ndc(P1, nf))) return;
+    float gxn = 0.f, gyn = 0.f, gzn = 0.f;
+    if (DX != 0) {
+        float dbx, dbz;
+        db_dp_2d(nv[0], nv[2], nf[0], nf[2], dbx, dbz);
+        gxn = gx * dbx; gzn = gx * dbz;
+    } else {
+        float dby, dbz;
+        db_dp_2d(nv[1], nv[2], nf[1], nf[2], dby, dbz);
+        gyn = gy * dby; gzn = gy * dbz;
+    }
+    add_mid_contrib(0.5f * (nx0 + nx1), 0.5f * (ny0 + ny1), P0, gxn, gyn, gzn, true, acc);
+}
+
 // Edge-gradient estimator of one pixel (rasterize.cu:663-892).  Pixel
 // buffers are addressed as base + y*W + x with `base` the view's first pixel;
 // posb holds the view's clip positions.  Returns the pixel's triangle (or -1)
@@ -184,51 +233,12 @@ __device__ __forceinline__ int edge_grad_pixel(int b, int y0, int x0, int H, int
                 float4 P1[3];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) P1[k] = load_vertex(posb, __ldg(tri + it1 * 3 + k));
-                float cz0, cw0;
-                if (intersect_triangle(ny0, nx0, P1[0], P1[1], P1[2], tb0, tb1, cz0, cw0)) {
-                    const float d0_it1 = cz0 / cw0;
-                    if (depth0 < d0_it1) {  // triangle intersection
-                        float nv[3], nf[3];
-                        if (tri_normal_ndc(P0, nv) && tri_normal_ndc(P1, nf)) {
-                            float gxn = 0.f, gyn = 0.f, gzn = 0.f;
-                            if (DX != 0) {
-                                float dbx, dbz;
-                                db_dp_2d(nv[0], nv[2], nf[0], nf[2], dbx, dbz);
-                                gxn = gx * dbx; gzn = gx * dbz;
-                            } else {
-                                float dby, dbz;
-                                db_dp_2d(nv[1], nv[2], nf[1], nf[2], dby, dbz);
-                                gyn = gy * dby; gzn = gy * dbz;
-                            }
-                            add_mid_contrib(mx, my, P0, gxn, gyn, gzn, true, acc);
-                        }
-                    }
-                }
+                intersection_contrib(P0, P1, depth0, nx0, ny0, nx1, ny1, DX, gx, gy, acc);
             } else if (it1 < 0 || depth0 < depth1) {  // active opacity edge
                 add_mid_contrib(mx, my, P0, gx, gy, 0.f, false, acc);
             }
         } else if (it1 < 0 || depth0 < depth1) {  // active geometric edge
-            int i0, i1;
-            float s0, s1;
-            if (find_edge_intersection(P0, nx0, ny0, nx1, ny1, i0, i1, s0, s1)) {
-                const float4 A = i0 == 0 ? P0[0] : (i0 == 1 ? P0[1] : P0[2]);
-                const float4 Bv = i1 == 0 ? P0[0] : (i1 == 1 ? P0[1] : P0[2]);
-                const float cx = s0 * A.x + s1 * Bv.x;
-                const float cy = s0 * A.y + s1 * Bv.y;
-                const float cw = s0 * A.w + s1 * Bv.w;
-                const float iw = 1.f / cw, iw2 = iw * iw;
-                const float gsum = gx * cx + gy * cy;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {  // static indices: no local-memory array
-                    const float s = k == i0 ? s0 : (k == i1 ? s1 : 0.f);
-                    if (k == i0 || k == i1) {
-                        acc.g[k * 4 + 0] += s * gx * iw;
-                        acc.g[k * 4 + 1] += s * gy * iw;
-                        acc.g[k * 4 + 3] += -s * gsum * iw2;
-                    }
-                }
-                acc.any = true;
-            }
+            edge_crossing_contrib(P0, nx0, ny0, nx1, ny1, gx, gy, acc);
         }
     }
     return it0;
@@ -511,6 +521,99 @@ __device__ __forceinline__ int edge_grad_pixel_staged(const EdgeHalo& h, int hid
         float ge_x, ge_y, ge_z;
         if (intersection_pair(f.P, tverts, h.it[p.n], f.depth, f.nx, f.ny, p.DX, p.gx, p.gy, ge_x, ge_y, ge_z))
             edge_midpoint(f, p.hx, p.hy, ge_x, ge_y, ge_z, acc);
+    }
+    return it0;
+}
+
+// The estimator of edge_grad_pixel from a staged tile, with its arithmetic: the
+// pairs are classified first (interior, silhouette, intersection; each marked pair's
+// adjoint kept in adj[e * kEdgeLanes]) and then evaluated kind by kind, round k of
+// a pass taking each lane's k-th pair of that kind, so that the lanes of a warp
+// run the same case together.  An interior pair is evaluated from its left or
+// bottom pixel and counted twice.  zhi of the tile is not used.
+__device__ __forceinline__ int edge_grad_pixel_tile(const EdgeHalo& h, int hidx, int y0, int x0, int H, int W,
+                                                    const float* __restrict__ posb, const int* __restrict__ tri,
+                                                    EdgeAccum& acc, float* adj, bool active) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc.g[k] = 0.f;
+    acc.any = false;
+    const int it0 = active ? h.it[hidx] : -1;
+    unsigned mid = 0u, geo = 0u, isect = 0u;  // pairs (bit e) of the midpoint, edge-crossing and intersection passes
+    const float nx0 = -1.f + 2.f * ((float)x0 + 0.5f) / (float)W;
+    const float ny0 = -1.f + 2.f * ((float)y0 + 0.5f) / (float)H;
+    float4 P0[3];
+    float depth0 = 0.f;
+    if (it0 >= 0) {
+        depth0 = h.dep[hidx];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) P0[k] = load_vertex(posb, __ldg(tri + it0 * 3 + k));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int DX = (e == 0) - (e == 1), DY = (e == 3) - (e == 2);
+            const int n = hidx + DX + DY * kHaloW, it1 = h.it[n];
+            if (it1 == kOutside) continue;
+            const bool interior = it1 == it0;
+            if (interior && (DX < 0 || DY < 0)) continue;  // counted by the neighbour
+            const float a = pair_adjoint(h, hidx, n);
+            if (a == 0.f) continue;
+            adj[e * kEdgeLanes] = a;
+            if (interior) {
+                mid |= 1u << e;
+                continue;
+            }
+            const float nx1 = -1.f + 2.f * ((float)(x0 + DX) + 0.5f) / (float)W;
+            const float ny1 = -1.f + 2.f * ((float)(y0 + DY) + 0.5f) / (float)H;
+            const float depth1 = h.dep[n];
+            const bool front = it1 < 0 || depth0 < depth1;
+            float tb0, tb1, cz1, cw1;
+            if (intersect_triangle(ny1, nx1, P0[0], P0[1], P0[2], tb0, tb1, cz1, cw1)) {
+                if (it1 >= 0 && depth1 < cz1 / cw1) isect |= 1u << e;
+                else if (front) mid |= 1u << e;  // active opacity edge
+            } else if (front) {  // active geometric edge
+                geo |= 1u << e;
+            }
+        }
+    }
+    const int nmid = __reduce_max_sync(0xffffffffu, (unsigned)__popc(mid));
+    for (int r = 0; r < nmid; ++r) {
+        if (mid == 0u) continue;
+        const int e = __ffs(mid) - 1;
+        mid &= mid - 1u;
+        const int DX = (e == 0) - (e == 1), DY = (e == 3) - (e == 2);
+        const float m = h.it[hidx + DX + DY * kHaloW] == it0 ? 2.f : 1.f;
+        const float gx = adj[e * kEdgeLanes] * (float)DX * (float)W / 2.f;
+        const float gy = adj[e * kEdgeLanes] * (float)DY * (float)H / 2.f;
+        const float nx1 = -1.f + 2.f * ((float)(x0 + DX) + 0.5f) / (float)W;
+        const float ny1 = -1.f + 2.f * ((float)(y0 + DY) + 0.5f) / (float)H;
+        add_mid_contrib(0.5f * (nx0 + nx1), 0.5f * (ny0 + ny1), P0, m * gx, m * gy, 0.f, false, acc);
+    }
+    const int ngeo = __reduce_max_sync(0xffffffffu, (unsigned)__popc(geo));
+    for (int r = 0; r < ngeo; ++r) {
+        if (geo == 0u) continue;
+        const int e = __ffs(geo) - 1;
+        geo &= geo - 1u;
+        const int DX = (e == 0) - (e == 1), DY = (e == 3) - (e == 2);
+        const float gx = adj[e * kEdgeLanes] * (float)DX * (float)W / 2.f;
+        const float gy = adj[e * kEdgeLanes] * (float)DY * (float)H / 2.f;
+        const float nx1 = -1.f + 2.f * ((float)(x0 + DX) + 0.5f) / (float)W;
+        const float ny1 = -1.f + 2.f * ((float)(y0 + DY) + 0.5f) / (float)H;
+        edge_crossing_contrib(P0, nx0, ny0, nx1, ny1, gx, gy, acc);
+    }
+    const int nisect = __reduce_max_sync(0xffffffffu, (unsigned)__popc(isect));
+    for (int r = 0; r < nisect; ++r) {
+        if (isect == 0u) continue;
+        const int e = __ffs(isect) - 1;
+        isect &= isect - 1u;
+        const int DX = (e == 0) - (e == 1), DY = (e == 3) - (e == 2);
+        const float gx = adj[e * kEdgeLanes] * (float)DX * (float)W / 2.f;
+        const float gy = adj[e * kEdgeLanes] * (float)DY * (float)H / 2.f;
+        const float nx1 = -1.f + 2.f * ((float)(x0 + DX) + 0.5f) / (float)W;
+        const float ny1 = -1.f + 2.f * ((float)(y0 + DY) + 0.5f) / (float)H;
+        const int it1 = h.it[hidx + DX + DY * kHaloW];
+        float4 P1[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) P1[k] = load_vertex(posb, __ldg(tri + it1 * 3 + k));
+        intersection_contrib(P0, P1, depth0, nx0, ny0, nx1, ny1, DX, gx, gy, acc);
     }
     return it0;
 }
