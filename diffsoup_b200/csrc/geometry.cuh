@@ -148,18 +148,18 @@ __device__ __forceinline__ bool block_surely_outside(float4 p0, float4 p1, float
     return a2 < -(t2 + 0x1p-19f * (m + tA));
 }
 
-// Per-triangle data of the block test of the rasterizer's staging pass:
-// e[k] = (ox, oy, oc, m) such that, for any block of pixel centres inside
-// the rect the record was built for, no centre can pass the reference's
-// coverage test when  max over the block of ox x + oy y + oc  <  -m  for
-// some k.  (ox, oy, oc) is the exact affine edge function E_k of
-// edge_terms (the w-products cancel), oriented so that the inside is
-// positive, and m bounds the difference between E_k and the reference's
-// FP32 value A_k, the evaluation of the rounded coefficients, and the
-// conditions under which surely_outside() rejects.  A record that
-// rejects nothing has oc = 1, m = 0.
+// Column bounds of a triangle, for the rasterizer's staging: on the pixel row of
+// NDC y, no pixel centre in a column left of lo0 = lo.x + lo.y y or lo1 = lo.z +
+// lo.w y, or right of hi0, hi1 (hi likewise) can pass the reference's coverage test, inside the
+// pixel rect that the record was built for.  Each bound is the line on which an
+// oriented affine edge function E_k (the w-products of edge_terms cancel) reaches
+// -m: there and beyond it, m covers the difference between E_k and the reference's FP32 value A_k
+// and the conditions under which surely_outside() rejects.  In columns it is c(y) = ca +
+// cb y, moved outwards by a hundredth of a pixel plus 2^-21 (|ca| + |cb|), more
+// than the rounding of ca, cb, their sum and the pixel centres.  An edge
+// almost parallel to the rows, or without a margin, bounds nothing.
 struct __align__(16) TriEdges {
-    float4 e[3];
+    float4 lo, hi;
 };
 
 // Builds the TriEdges of a triangle over the pixel-centre NDC rect
@@ -176,11 +176,16 @@ struct __align__(16) TriEdges {
 //    rejects (surely_outside); margin t_k + 2^-99 max|A|.
 //  * k = 2: A2 of the opposite sign with |A2| > 2^-20 (|A| + |A0| + |A1|)
 //    rejects; margin t_2 + 2^-19 (max|A| + max|A0| + max|A1|).
-//  * The block maximum is computed in FP32 from the rounded coefficients,
-//    within 2^-22 (|ox| + |oy| + |oc|) for |x|, |y| <= 1; margin 2^-21 of it.
+//  * The coefficients are rounded to FP32 before the division: margin 2^-21
+//    (|ox| + |oy| + |oc|).
+// width: columns of the view.
 __device__ inline TriEdges tri_edges_over_rect(float4 p0, float4 p1, float4 p2, float xa, float xb, float ya,
-                                               float yb) {
+                                               float yb, int width) {
     TriEdges out;
+    out.lo = make_float4(-1e9f, 0.f, -1e9f, 0.f);
+    out.hi = make_float4(1e9f, 0.f, 1e9f, 0.f);
+    const float half_w = 0.5f * (float)width;
+    int nlo = 0, nhi = 0;
     const double4 P[3] = {make_double4(p0.x, p0.y, p0.z, p0.w), make_double4(p1.x, p1.y, p1.z, p1.w),
                           make_double4(p2.x, p2.y, p2.z, p2.w)};
     double Qx[3], Qy[3];
@@ -220,23 +225,21 @@ __device__ inline TriEdges tri_edges_over_rect(float4 p0, float4 p1, float4 p2, 
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const double m = t[k] + (k == 2 ? m2 : m01) + 0x1p-21 * (fabs(ax[k]) + fabs(ay[k]) + fabs(c[k]));
-        const float mf = (float)(m * (1.0 + 0x1p-20));
-        const bool ok = sgn != 0.0 && isfinite(m) && isfinite(mf);
-        out.e[k] = ok ? make_float4((float)(sgn * ax[k]), (float)(sgn * ay[k]), (float)(sgn * c[k]), mf)
-                      : make_float4(0.f, 0.f, 1.f, 0.f);
-    }
-    return out;
-}
-
-// True when the TriEdges record proves that no pixel centre of the block
-// [xa, xb] x [ya, yb] (inside the record's rect) is covered.
-__device__ __forceinline__ bool edges_reject_block(const TriEdges& r, float xa, float xb, float ya, float yb) {
-    bool out = false;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float4 e = r.e[k];
-        const float v = fmaf(e.x, e.x > 0.f ? xb : xa, fmaf(e.y, e.y > 0.f ? yb : ya, e.z));
-        out = out || v < -e.w;
+        const float ox = (float)(sgn * ax[k]), oy = (float)(sgn * ay[k]), ocm = (float)(sgn * c[k] + m * (1.0 + 0x1p-20));
+        const float inv = __fdiv_rn(half_w, ox);
+        const float ca = __fmaf_rn(-ocm, inv, half_w - 0.5f), cb = -oy * inv;
+        const float eps = 0.01f + 0x1p-21f * (fabsf(ca) + fabsf(cb));
+        if (sgn == 0.0 || !isfinite(m) || !(fabsf(ox) > 1e-30f) || !(eps <= 1e8f)) continue;
+        // a triangle has one or two bounds on a side; a third (rounding of a degenerate one) is left out
+        if (ox > 0.f) {
+            if (nlo == 0) { out.lo.x = ca - eps; out.lo.y = cb; }
+            else if (nlo == 1) { out.lo.z = ca - eps; out.lo.w = cb; }
+            ++nlo;
+        } else {
+            if (nhi == 0) { out.hi.x = ca + eps; out.hi.y = cb; }
+            else if (nhi == 1) { out.hi.z = ca + eps; out.hi.w = cb; }
+            ++nhi;
+        }
     }
     return out;
 }

@@ -6,10 +6,10 @@
 // (src/cuda/rasterize.cu:139-400).  Here each (view, triangle) is binned into
 // the 16x16 screen tiles its rect (rasterize.cu:43-137) overlaps, and each
 // tile's list is sorted by the triangles' near-depth bound.  A work item is
-// one 8x4 pixel block of a tile, owned by one warp: the warp filters the
-// tile's triangle boxes 32 at a time (rect overlap, depth bound), stages the
-// survivors' vertices in its own shared memory, and every lane resolves its
-// pixel's depth test in registers.  Warps never wait for each other: no
+// one 8x4 pixel block of a tile, owned by one warp: the warp takes the tile's
+// entries 32 at a time (rect overlap, depth bound, pixels that may be covered),
+// stages the survivors' vertices in its own shared memory, and every lane walks
+// its own pixel's candidates and resolves the depth test in registers.  Warps never wait for each other: no
 // fragment list, no CTA barrier, no global atomics, one 16-byte store per
 // pixel.
 //
@@ -221,11 +221,10 @@ __global__ void __launch_bounds__(kThreads) bin_setup_kernel(int B, const ds_vie
     if (!live) return;
     const uint64_t m = ntiles <= 64 ? s_mask[threadIdx.x] : 0ull;
     TriEdges te;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) te.e[k] = make_float4(0.f, 0.f, 1.f, 0.f);
+    te.lo = te.hi = make_float4(0.f, 0.f, 0.f, 0.f);  // not read: the rect is empty
     if (ntiles > 0)
         te = tri_edges_over_rect(v.p0, v.p1, v.p2, pix_ndc(r.x0, vd.W), pix_ndc(r.x1 - 1, vd.W), pix_ndc(r.y0, vd.H),
-                                 pix_ndc(r.y1 - 1, vd.H));
+                                 pix_ndc(r.y1 - 1, vd.H), vd.W);
     TriNdc q;
     q.a = make_float4(v.p0.x / v.p0.w, v.p0.y / v.p0.w, v.p1.x / v.p1.w, v.p1.y / v.p1.w);
     q.b = make_float4(v.p2.x / v.p2.w, v.p2.y / v.p2.w, __uint_as_float((uint32_t)m),
@@ -528,78 +527,6 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-// Candidates of one group of up to 32 list entries staged in warp-private
-// shared memory, in list order.
-struct WarpStage {
-    TriVerts v[32];
-    TriBox box[32];
-    int t[32];
-    unsigned lanes[32];  // lanes of the block whose (valid) pixel lies inside the candidate's rect
-};
-
-// Lanes of the block whose pixel lies inside the pixel rect r (lane l =
-// pixel (l mod bw, l div bw) of the block).
-__device__ __forceinline__ unsigned rect_lanes(const TriBox& r, const BlockGeom& g) {
-    const int cx0 = max((int)r.x0 - g.wx0, 0), cx1 = min((int)r.x1 - g.wx0, g.bw);
-    const int cy0 = max((int)r.y0 - g.wy0, 0), cy1 = min((int)r.y1 - g.wy0, g.bh);
-    if (cx0 >= cx1 || cy0 >= cy1) return 0u;
-    const unsigned row = ((1u << cx1) - 1u) & ~((1u << cx0) - 1u);  // cx1 <= bw <= 16
-    // one bit per block row, at the row's first lane: 0xffffffff / (2^bw - 1)
-    const unsigned rows = g.bw == 8 ? 0x01010101u : (g.bw == 16 ? 0x00010001u : 0x11111111u);
-    const int hi = cy1 * g.bw;  // <= 32
-    const unsigned keep = (hi >= 32 ? ~0u : (1u << hi) - 1u) & ~((1u << (cy0 * g.bw)) - 1u);
-    return row * (rows & keep);  // the row bits repeated on the kept rows (no carries)
-}
-
-// Loads entries [g0, g0+32) of the work item's range, keeps those whose box
-// meets the block, whose depth bound passes `zcut` (zlo <= zcut) and whose
-// edge record does not prove the block uncovered, stages them, and returns
-// how many were staged.  *head_zlo receives the zlo of the group's first
-// entry (the smallest, when the list is ordered).
-__device__ __forceinline__ int stage_group(const BlockGeom& g, int64_t g0, const TriBox* __restrict__ boxes,
-                                           const TriVerts* __restrict__ verts, const TriEdges* __restrict__ edges,
-                                           const ListEntry* __restrict__ list, int T, float zcut, WarpStage& st,
-                                           float* head_zlo) {
-    const int lane = threadIdx.x & 31;
-    const int64_t e = g0 + lane;
-    const bool in = e < g.end;
-    int ri = 0;
-    TriBox bx;
-    bx.y0 = bx.y1 = bx.x0 = bx.x1 = 0;
-    bx.zlo = INFINITY; bx.zhi = INFINITY;
-    if (in) {
-        if (g.exhaustive) {
-            ri = (int)e;
-            bx = boxes[ri];
-        } else {
-            const int4 le = __ldg(reinterpret_cast<const int4*>(list + e));
-            ri = le.w;
-            bx.y0 = (short)(le.x & 0xffff); bx.y1 = (short)(le.x >> 16);
-            bx.x0 = (short)(le.y & 0xffff); bx.x1 = (short)(le.y >> 16);
-            bx.zlo = __int_as_float(le.z);
-        }
-    }
-    *head_zlo = __shfl_sync(0xffffffffu, bx.zlo, 0);
-    bool c = in && box_overlaps(bx, g) && bx.zlo <= zcut;
-    if (c) {
-        // pixel-centre extents of the block (clamped to the view)
-        const float xa = pix_ndc(g.wx0, g.W), xb = pix_ndc(min(g.wx0 + g.bw - 1, g.W - 1), g.W);
-        const float ya = pix_ndc(g.wy0, g.H), yb = pix_ndc(min(g.wy0 + g.bh - 1, g.H - 1), g.H);
-        c = !edges_reject_block(edges[ri], xa, xb, ya, yb);
-    }
-    const unsigned mask = __ballot_sync(0xffffffffu, c);
-    const unsigned valid = __ballot_sync(0xffffffffu, g.valid);
-    if (c) {
-        const int k = __popc(mask & ((1u << lane) - 1u));
-        st.v[k] = verts[ri];
-        st.box[k] = bx;
-        st.t[k] = ri - g.b * T;
-        st.lanes[k] = rect_lanes(bx, g) & valid;
-    }
-    __syncwarp();
-    return __popc(mask);
-}
-
 // Per-warp buffer of the fragment records of one 8x4 block (REC kernels).
 constexpr int kRecCap = 192;
 
@@ -664,17 +591,109 @@ __device__ __forceinline__ void flush_records(const RecordStore& rs, const WarpR
     cfill += at;
 }
 
-// Forward: depth test with stochastic opacity.  Each warp walks the
-// triangles of its block front to back (the tile list is sorted by zlo) and
-// stops once the next triangle's depth bound lies behind the winner of every
-// lane: no later triangle can improve a key (the bound's margin keeps
-// bits(z+2) strictly larger).  Within a triangle, the divisions run only when
-// some lane survives the cheap edge-sign test.
+// Candidates of one group of 32 list entries, by the entry's place in the group,
+// and the NDC y of the block's rows.
+struct RasterStage {
+    TriVerts v[32];
+    float zlo[32];
+    int t[32];
+    float row_y[8];
+};
+
+// Lanes of the block (lane l = pixel (l mod bw, l div bw)) whose pixel centre the
+// triangle may cover: its pixel rect, cut row by row to its column bounds.
+__device__ __forceinline__ unsigned cover_lanes(const TriBox& r, const TriEdges& te, const BlockGeom& g,
+                                                const float* row_y) {
+    const float lo0 = (float)max((int)r.x0, g.wx0), hi0 = (float)(min((int)r.x1, g.wx0 + g.bw) - 1);
+    const int y0 = max((int)r.y0 - g.wy0, 0), y1 = min((int)r.y1 - g.wy0, g.bh);
+    unsigned lanes = 0u;
+    for (int y = y0; y < y1; ++y) {
+        const float ny = row_y[y];
+        const float lo = fmaxf(lo0, fmaxf(fmaf(te.lo.y, ny, te.lo.x), fmaf(te.lo.w, ny, te.lo.z)));
+        const float hi = fminf(hi0, fminf(fmaf(te.hi.y, ny, te.hi.x), fmaf(te.hi.w, ny, te.hi.z)));
+        // whole columns inside [lo, hi], relative to the block (lo >= its first, hi <= its last column)
+        const int a = (int)ceilf(fminf(lo, hi0 + 1.f)) - g.wx0, c = (int)floorf(fmaxf(hi, lo0 - 1.f)) - g.wx0;
+        if (a <= c) lanes |= ((2u << c) - (1u << a)) << (y * g.bw);
+    }
+    return lanes;
+}
+
+// Transposes the 32x32 bit matrix held as one row per lane: bit l of lane k's word
+// becomes bit k of lane l's.
+__device__ __forceinline__ unsigned warp_transpose(unsigned m) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned low = 0xffffffffu / ((1u << o) + 1u);  // the low halves of the 2 o-bit fields
+        const unsigned other = __shfl_xor_sync(0xffffffffu, m, o);
+        m = (lane & o) ? (m & ~low) | ((other >> o) & low) : (m & low) | ((other << o) & ~low);
+    }
+    return m;
+}
+
+// Loads entries [g0, g0 + 32) of the work item's range, stages those whose box
+// meets the block, whose depth bound passes `zcut` and that may cover one of its
+// valid pixels, and returns the calling lane's pixel's candidates as a mask over
+// the group.  *head_zlo receives the zlo of the group's first entry (the
+// smallest, when the list is ordered).
+__device__ __forceinline__ unsigned stage_pixels(const BlockGeom& g, int64_t g0, const TriBox* __restrict__ boxes,
+                                                 const TriVerts* __restrict__ verts,
+                                                 const TriEdges* __restrict__ edges,
+                                                 const ListEntry* __restrict__ list, int T, float zcut, unsigned valid,
+                                                 RasterStage& st, float* head_zlo) {
+    const int lane = threadIdx.x & 31;
+    const int64_t e = g0 + lane;
+    const bool in = e < g.end;
+    int ri = 0;
+    TriBox bx;
+    bx.y0 = bx.y1 = bx.x0 = bx.x1 = 0;
+    bx.zlo = INFINITY; bx.zhi = INFINITY;
+    if (in) {
+        if (g.exhaustive) {
+            ri = (int)e;
+            bx = boxes[ri];
+        } else {
+            const int4 le = __ldg(reinterpret_cast<const int4*>(list + e));
+            ri = le.w;
+            bx.y0 = (short)(le.x & 0xffff); bx.y1 = (short)(le.x >> 16);
+            bx.x0 = (short)(le.y & 0xffff); bx.x1 = (short)(le.y >> 16);
+            bx.zlo = __int_as_float(le.z);
+        }
+    }
+    *head_zlo = __shfl_sync(0xffffffffu, bx.zlo, 0);
+    unsigned lanes = 0u;
+    if (in && box_overlaps(bx, g) && bx.zlo <= zcut) lanes = cover_lanes(bx, edges[ri], g, st.row_y) & valid;
+    if (lanes != 0u) {
+        st.v[lane] = verts[ri];
+        st.zlo[lane] = bx.zlo;
+        st.t[lane] = ri - g.b * T;
+    }
+    __syncwarp();
+    return warp_transpose(lanes);
+}
+
+// Forward: depth test with stochastic opacity.  A warp takes the triangles of
+// its block front to back (the tile list is sorted by zlo), 32 list entries at a time:
+// staging finds for every entry the pixels it may cover (cover_lanes, one entry a
+// lane), and then every lane walks its own pixel's candidates in order, so a pass
+// evaluates up to 32 different (pixel, triangle) pairs.  A lane stops once its next
+// triangle's depth bound lies behind its winner, and the warp once the next
+// group's lies behind every lane's: no later triangle can improve a key (the bound's margin
+// keeps bits(z+2) strictly larger).
+//
+// Issue slots bound the kernel, and a triangle covers 7 of a block's 32 pixels: with the
+// warp on one triangle at a time a block took 7.5 passes of coverage, opacity and
+// threshold and 10 of edge functions; now its passes are the most candidates of
+// one pixel, about 4.  8 views of 800x800 (15,000 triangles, records kept): 367 ->
+// 269 us, 6 uneven views 282 -> 227 us, one 1200x1200 view without records
+// 74 -> 61 us.  (Four 4x2 sub-blocks of a warp with a candidate each took 6.5
+// passes, not worth their staging; 3 or 5 CTAs per SM, 304 and 302 us; drawing the next work
+// item ahead, 272 us.)
 //
 // REC: also keeps every fragment whose depth key does not lie behind the
 // lane's current winner.  Winner keys only decrease, and every fragment at
-// or in front of a lane's final surface has zlo <= that depth <= the warp's
-// bound at every point of the walk, so the walk meets and keeps all of them;
+// or in front of a lane's final surface has zlo <= that depth <= the lane's winner's
+// at every point of the walk, so the walk meets and keeps all of them;
 // at the end of the block those behind the final surface are dropped.
 #ifndef DSB_RASTER_MIN_CTAS
 #define DSB_RASTER_MIN_CTAS 4  // resident 8-warp CTAs per SM the register budget is sized for (64 registers)
@@ -687,10 +706,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
     const int* __restrict__ sorted, const ListEntry* __restrict__ list, int64_t capacity, int level, int S,
     const float* __restrict__ alpha_src, int thr_mode, float thr_const, const uint64_t* __restrict__ rng, int* work, float* __restrict__ rast,
     RecordStore rs, int bwl) {
-    __shared__ WarpStage s_stage[kWarpsPerCta];
+    __shared__ RasterStage s_stage[kWarpsPerCta];
     __shared__ WarpRecs s_rec[REC ? kWarpsPerCta : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpStage& st = s_stage[warp];
+    RasterStage& st = s_stage[warp];
     WarpRecs& R = s_rec[REC ? warp : 0];
     uint64_t seed = 0;
     uint32_t iter = 0;
@@ -704,40 +723,36 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
             continue;
         }
         const float ndc_x = pix_ndc(g.px, g.W), ndc_y = pix_ndc(g.py, g.H);
+        if ((lane & (g.bw - 1)) == 0) st.row_y[lane >> bwl] = ndc_y;
+        const unsigned valid = __ballot_sync(0xffffffffu, g.valid);
+        __syncwarp();
         const PhiloxPixel php = philox_pixel(seed, iter, (uint32_t)g.b, (uint32_t)(g.py * g.W + g.px));
         unsigned long long best = ~0ull;
         float bb0 = 0.f, bb1 = 0.f, bz = 0.f;
-        float bz_cut = INFINITY;  // the winner's depth, +inf while the lane has none
+        float bz_cut = g.valid ? INFINITY : -INFINITY;  // the winner's depth, +inf while a valid lane has none
         int nrec = 0;
-        // max over the warp of the lanes' winning depth (+inf while a valid lane has none)
-        float warp_far = warp_max(g.valid ? INFINITY : -INFINITY);
-        bool all_won = false;  // every valid lane has a winner (before that, warp_far stays +inf)
         for (int64_t g0 = g.begin; g0 < g.end; g0 += 32) {
             float head;
-            const int nc = stage_group(g, g0, boxes, verts, edges, list, T, warp_far, st, &head);
+            const float warp_far = warp_max(bz_cut);  // the farthest winner
+            unsigned todo = stage_pixels(g, g0, boxes, verts, edges, list, T, warp_far, valid, st, &head);
             if (g.ordered && head > warp_far) break;  // this group and all later ones lie behind
-            for (int k = 0; k < nc; ++k) {
-                if (st.box[k].zlo > warp_far) {
-                    if (g.ordered) break;
-                    continue;
-                }
-                const float4 p0 = st.v[k].p0, p1 = st.v[k].p1, p2 = st.v[k].p2;
-                const TriBox r = st.box[k];
-                // lanes inside the rect whose winner does not lie in front of the triangle: zlo's
-                // margin exceeds the rounding of z + 2, so with zlo > bz every fragment's depth key
-                // lies strictly behind the winner's (neither a winner nor a record)
-                const bool near = ((st.lanes[k] >> lane) & 1u) && !(r.zlo > bz_cut);
+            while (__any_sync(0xffffffffu, todo != 0u)) {
+                const int k = todo != 0u ? __ffs(todo) - 1 : 0;
+                // the winner does not lie in front of the triangle: zlo's margin exceeds the rounding of
+                // z + 2, so with zlo > bz every fragment's depth key lies strictly behind the winner's
+                // (neither a winner nor a record)
+                const bool near = todo != 0u && !(st.zlo[k] > bz_cut);
+                todo = !near && g.ordered ? 0u : todo & (todo - 1u);
                 if (!__any_sync(0xffffffffu, near)) continue;  // warp-uniform
-                float A0, A1, A2, A;
-                edge_terms(ndc_y, ndc_x, p0, p1, p2, A0, A1, A2, A);
-                const bool cand = near && !surely_outside(A0, A1, A2, A);
-                if (!__any_sync(0xffffffffu, cand)) continue;  // warp-uniform
-                bool improved = false, rec = false;
+                bool rec = false;
                 float b0 = 0.f, b1 = 0.f, depth = 0.f;
                 const uint32_t t = (uint32_t)st.t[k];
-                if (cand) {
+                if (near) {
+                    const float4 p0 = st.v[k].p0, p1 = st.v[k].p1, p2 = st.v[k].p2;
+                    float A0, A1, A2, A;
+                    edge_terms(ndc_y, ndc_x, p0, p1, p2, A0, A1, A2, A);
                     float z, w;
-                    if (finish_coverage(A0, A1, A, p0, p1, p2, b0, b1, z, w)) {
+                    if (!surely_outside(A0, A1, A2, A) && finish_coverage(A0, A1, A, p0, p1, p2, b0, b1, z, w)) {
                         depth = __fdiv_rn(z, w);
                         if (depth >= -1.f && depth <= 1.f) {
                             const unsigned long long key = depth_key(depth, t);
@@ -746,17 +761,14 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
                             // surface is dropped (the winner's depth itself can grow within one
                             // bits(z+2) step when a lower triangle index takes a tie)
                             if (REC) rec = (key >> 32) <= (best >> 32);
-                            if (depth > -1.f) {
-                                if (key < best) {
-                                    const float alpha = interp_level(b0, b1, level, alpha_src + (size_t)t * S);
-                                    // Philox thresholds lie in [0, 1): an opacity of 1 passes without a draw
-                                    const bool pass = thr_mode == 1
-                                                          ? alpha >= 1.f || !(alpha < philox_uniform_tri(php, seed, t))
-                                                          : !(alpha < thr_const);
-                                    if (pass) {
-                                        best = key; bb0 = b0; bb1 = b1; bz = depth; bz_cut = depth;
-                                        improved = true;
-                                    }
+                            if (depth > -1.f && key < best) {
+                                const float alpha = interp_level(b0, b1, level, alpha_src + (size_t)t * S);
+                                // Philox thresholds lie in [0, 1): an opacity of 1 passes without a draw
+                                const bool pass = thr_mode == 1
+                                                      ? alpha >= 1.f || !(alpha < philox_uniform_tri(php, seed, t))
+                                                      : !(alpha < thr_const);
+                                if (pass) {
+                                    best = key; bb0 = b0; bb1 = b1; bz = depth; bz_cut = depth;
                                 }
                             }
                         }
@@ -772,10 +784,6 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
                         }
                         nrec += __popc(m);
                     }
-                }
-                if (__any_sync(0xffffffffu, improved)) {
-                    if (!all_won) all_won = __all_sync(0xffffffffu, !g.valid || best != ~0ull);
-                    if (all_won) warp_far = warp_max(!g.valid ? -INFINITY : bz);
                 }
             }
             __syncwarp();  // the stage is rewritten by the next group
@@ -876,7 +884,8 @@ __global__ void __launch_bounds__(kRecChunk) aux_records_kernel(RecordStore rs, 
 // lane's surface are never staged.  A fragment's three contributions go
 // straight to memory: about one fragment a pixel is in front of its surface, far below
 // the atomics' rate (summing a warp's contributions in shared memory first, with its
-// compare-and-swap loops, took 124 us against 79 us for two views of 803x601).
+// compare-and-swap loops, took 124 us against 79 us for two views of 803x601; per-pixel
+// candidates as in the rasterizer then gave 65 us).
 // With item_list, only the blocks listed there (*item_count of them) are processed.
 __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
     int B, const ds_view_desc* __restrict__ views, int num_tiles, int T, const TriBox* __restrict__ boxes,
@@ -886,15 +895,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
     const float* __restrict__ color, const float* __restrict__ target, const float* __restrict__ rast, float scale,
     const int* __restrict__ item_list, const int* __restrict__ item_count, int* work,
     float* __restrict__ grad_alpha_src, int bwl) {
-    __shared__ WarpStage s_stage[kWarpsPerCta];
+    __shared__ RasterStage s_stage[kWarpsPerCta];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpStage& st = s_stage[warp];
+    RasterStage& st = s_stage[warp];
     const int items = item_list ? *item_count : num_tiles * kBlocksPerTile;
     for (int n = warp_next(work, items); n < items; n = warp_next(work, items)) {
         const int item = item_list ? item_list[n] : n;
         const BlockGeom g = block_geometry(item, B, views, T, offsets, sorted, capacity, bwl);
         if (g.begin >= g.end) continue;  // no triangle, no fragment
         const float ndc_x = pix_ndc(g.px, g.W), ndc_y = pix_ndc(g.py, g.H);
+        if ((lane & (g.bw - 1)) == 0) st.row_y[lane >> bwl] = ndc_y;
+        const unsigned valid = __ballot_sync(0xffffffffu, g.valid);
+        __syncwarp();
         int tp = -1;
         float zp = 0.f, loss = 0.f;
         if (g.valid) {
@@ -907,33 +919,24 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
                 loss = color[g.pix];  // caller passes the per-pixel sum |c - target| directly
             }
         }
-        // farthest surface of the block (+inf where a valid pixel is empty)
-        const float warp_far = warp_max(!g.valid ? -INFINITY : (tp >= 0 ? zp : INFINITY));
+        // the surface's depth (+inf where a valid pixel is empty) and the block's farthest
+        const float z_cut = !g.valid ? -INFINITY : (tp >= 0 ? zp : INFINITY);
+        const float warp_far = warp_max(z_cut);
         for (int64_t g0 = g.begin; g0 < g.end; g0 += 32) {
             float head;
-            const int nc = stage_group(g, g0, boxes, verts, edges, list, T, warp_far, st, &head);
+            unsigned todo = stage_pixels(g, g0, boxes, verts, edges, list, T, warp_far, valid, st, &head);
             if (g.ordered && head > warp_far) break;
-            for (int k = 0; k < nc; ++k) {
-                const TriBox r = st.box[k];
+            while (__any_sync(0xffffffffu, todo != 0u)) {
+                const int k = todo != 0u ? __ffs(todo) - 1 : 0;
+                // the pixel's surface does not lie in front of the triangle
+                const bool near = todo != 0u && !(st.zlo[k] > z_cut);
+                todo = !near && g.ordered ? 0u : todo & (todo - 1u);
+                if (!near) continue;
                 const int t = st.t[k];
                 const float4 p0 = st.v[k].p0, p1 = st.v[k].p1, p2 = st.v[k].p2;
-                // lanes inside the rect whose surface does not lie in front of the triangle
-                const bool near = ((st.lanes[k] >> lane) & 1u) && !(tp >= 0 && r.zlo > zp);
-                if (!__any_sync(0xffffffffu, near)) continue;  // warp-uniform
-                float A0, A1, A2, A;
-                edge_terms(ndc_y, ndc_x, p0, p1, p2, A0, A1, A2, A);
-                bool hit = near && !surely_outside(A0, A1, A2, A);
-                if (!__any_sync(0xffffffffu, hit)) continue;  // warp-uniform
-                float b0 = 0.f, b1 = 0.f;
-                if (hit) {
-                    float z, w;
-                    hit = finish_coverage(A0, A1, A, p0, p1, p2, b0, b1, z, w);
-                    if (hit) {
-                        const float depth = __fdiv_rn(z, w);
-                        hit = depth >= -1.f && depth <= 1.f && !(tp >= 0 && depth > zp);
-                    }
-                }
-                if (hit) aux_scatter(b0, b1, level, S, alpha_src, t, loss, tp >= 0 && t == tp, scale, grad_alpha_src);
+                float b0, b1, depth;
+                if (fragment_at(ndc_y, ndc_x, p0, p1, p2, b0, b1, depth) && !(tp >= 0 && depth > zp))
+                    aux_scatter(b0, b1, level, S, alpha_src, t, loss, tp >= 0 && t == tp, scale, grad_alpha_src);
             }
             __syncwarp();
         }

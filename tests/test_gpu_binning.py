@@ -20,7 +20,7 @@ def al(n):
 def lists_of(b):
     """Per tile the (zlo, record) pairs in list order, and the tile's sorted flag, from the bins' workspace."""
     ws, n, nt = b.workspace.cpu().numpy(), b.B * b.T, b.num_tiles
-    o = al(16 * n) + al(48 * n) + al(32 * n) + al(48 * n) + al(4 * nt)
+    o = al(16 * n) + al(48 * n) + al(32 * n) + al(32 * n) + al(4 * nt)
     off = ws[o:o + 8 * (nt + 1)].view(np.int64)
     o += al(8 * (nt + 1)) + al(4 * nt)
     flags = ws[o:o + 4 * nt].view(np.int32)
