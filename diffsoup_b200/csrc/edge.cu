@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kThreads) edge_grad_kernel(int B, int H, int W
 
 // The same for three channels: one CTA per 16x16 tile of a view, its pixels and
 // their border staged in shared memory, the covered pixels compacted onto the
-// first threads, pairs evaluated kind by kind (edge_grad_pixel_tile) and runs of
+// first threads triangle by triangle, pairs evaluated kind by kind (edge_grad_pixel_tile) and runs of
 // one triangle in a warp summed before the atomics.  Two views of 803x601, 15,000
 // triangles: 189 -> 101 us (one thread per pixel ran 13.5 of 32 lanes on 98
 // registers and 12 atomics a pixel).
@@ -78,17 +78,8 @@ __global__ void __launch_bounds__(kEdgeTileThreads, 3) edge_grad_tile_kernel(
 #pragma unroll
         for (int k = 0; k < 3; ++k) { h.c[k][i] = cc[k]; h.g[k][i] = gg[k]; }
     }
-    const unsigned m = __ballot_sync(0xffffffffu, cov);
-    if (lane == 0) s_warp_n[warp] = __popc(m);
     __syncthreads();
-    int n = 0, off = 0;
-#pragma unroll
-    for (int w = 0; w < kEdgeTileThreads / 32; ++w) {
-        off += w < warp ? s_warp_n[w] : 0;
-        n += s_warp_n[w];
-    }
-    if (cov) s_pix[off + __popc(m & ((1u << lane) - 1u))] = (short)threadIdx.x;
-    __syncthreads();
+    const int n = edge_tile_order(h, s_pix, s_warp_n);
     if (warp * 32 >= n) return;  // warp-uniform: no covered pixel left for this warp
     const bool active = (int)threadIdx.x < n;
     const int src = active ? s_pix[threadIdx.x] : 0;

@@ -313,6 +313,36 @@ struct EdgeHalo {
     float g[3][kHaloN];
 };
 
+// The order in which a CTA of 256 threads takes the tile's covered pixels: fills
+// s_pix (pixel = row * 16 + column) and returns their number.  A warp brings 8x4
+// pixels, grouped by triangle, so that pixels of one triangle follow each other.
+__device__ __forceinline__ int edge_tile_order(const EdgeHalo& h, short* s_pix, int* s_warp_n) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cx = (warp & 1) * 8 + (lane & 7), cy = (warp >> 1) * 4 + (lane >> 3);
+    const int it = h.it[(cy + 1) * kHaloW + cx + 1];
+    const bool cov = it >= 0;  // a triangle (not background, not outside)
+    const unsigned m = __ballot_sync(0xffffffffu, cov);
+    const unsigned peers = __match_any_sync(0xffffffffu, cov ? it : -1);
+    int rank = 0;  // place among the warp's covered pixels
+    for (unsigned rest = m, before = 0; rest != 0;) {
+        const unsigned group = __shfl_sync(0xffffffffu, peers, __ffs(rest) - 1);
+        if ((group >> lane) & 1u) rank = (int)before + __popc(group & ((1u << lane) - 1u));
+        before += __popc(group);
+        rest &= ~group;
+    }
+    if (lane == 0) s_warp_n[warp] = __popc(m);
+    __syncthreads();
+    int off = 0, n = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        off += w < warp ? s_warp_n[w] : 0;
+        n += s_warp_n[w];
+    }
+    if (cov) s_pix[off + rank] = (short)(cy * DS_TILE + cx);
+    __syncthreads();
+    return n;
+}
+
 // One pixel pair of the staged estimator: the pixel's frame (its triangle's
 // clip vertices, the edge functions at its centre and their NDC
 // derivatives) and the pair's neighbour offset.

@@ -442,8 +442,12 @@ __global__ void __launch_bounds__(kThreads) project_backward_kernel(int B, int V
 // mostly share a triangle along a row: a segmented warp reduction sums runs
 // of equal triangles before one FP64 atomic per vertex component.  Only
 // covered pixels have a contribution, so after staging the tile's covered
-// pixels are compacted (row-major order kept) onto the CTA's first threads:
-// warps run full of covered pixels and the warps left without one exit.
+// pixels are compacted onto the CTA's first threads, triangle by triangle
+// (edge_tile_order): warps run full of covered pixels and the warps left
+// without one exit.  In row order, where stochastic opacity alternates
+// surfaces from pixel to pixel, half of a dense scene's time went to the atomics of its
+// short runs: 200,000 triangles in 3 full-HD views 707 -> 387 us, 6 uneven views
+// 292 -> 224 us, 8 views of 800x800 268 -> 265 us.
 constexpr int kEdgeThreads = DS_TILE * DS_TILE;
 #ifndef DSB_EDGE_MIN_CTAS
 #define DSB_EDGE_MIN_CTAS 4  // resident 8-warp CTAs per SM the register budget is sized for (64 registers)
@@ -496,22 +500,7 @@ __global__ void __launch_bounds__(kEdgeThreads, DSB_EDGE_MIN_CTAS) edge_step_ker
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ short s_pix[kEdgeThreads];
     __shared__ int s_warp_n[kEdgeThreads / 32];
-    int n = 0;
-    {
-        const int cy = threadIdx.x / DS_TILE, cx = threadIdx.x % DS_TILE;
-        const bool cov = h.it[(cy + 1) * kHaloW + cx + 1] >= 0;  // a triangle (not background, not outside)
-        const unsigned m = __ballot_sync(0xffffffffu, cov);
-        if (lane == 0) s_warp_n[warp] = __popc(m);
-        __syncthreads();
-        int off = 0;
-#pragma unroll
-        for (int w = 0; w < kEdgeThreads / 32; ++w) {
-            off += w < warp ? s_warp_n[w] : 0;
-            n += s_warp_n[w];
-        }
-        if (cov) s_pix[off + __popc(m & ((1u << lane) - 1u))] = (short)threadIdx.x;
-        __syncthreads();
-    }
+    const int n = edge_tile_order(h, s_pix, s_warp_n);
     if (warp * 32 >= n) return;  // warp-uniform: no covered pixel left for this warp
     const bool active = (int)threadIdx.x < n;
     const int src = active ? s_pix[threadIdx.x] : 0;
