@@ -530,33 +530,49 @@ static SplitWs carve_split(void* ws, int M, size_t* bytes) {
     return w;
 }
 
+static float bits_float(unsigned b) { float f; std::memcpy(&f, &b, 4); return f; }
+static unsigned float_bits(float f) { unsigned b; std::memcpy(&b, &f, 4); return b; }
+
+// Bins of the bits [lo, hi): the smallest width that kSplitBins of them cover.
+static SplitHist split_bins(int* bins, unsigned lo, unsigned hi) {
+    SplitHist h{bins, lo, hi, 0};
+    while (((hi - lo - 1) >> h.shift) >= (unsigned)kSplitBins) ++h.shift;
+    return h;
+}
+
 // One counting pass under `plan` (quotas when given): per-face counts into
 // w.counts, their exclusive scan into offsets [M+1]; returns the total, or -1
-// when a family or the call exceeded the limits.
+// when a family or the call exceeded the limits.  hist: also counts the splits'
+// keys into its bins and reads them back into bins_host.
 static int64_t count_pass(const SplitParams& P, SplitPlan plan, const int* quota, int M, const float* verts,
                           const int* faces, const int* valid, int64_t* offsets, const SplitWs& w, cudaStream_t st,
-                          int* rc) {
+                          int* rc, SplitHist hist = SplitHist{}, int* bins_host = nullptr) {
     *rc = DS_OK;
-    if (cudaMemsetAsync(w.total, 0, 16, st) != cudaSuccess) { *rc = check_launch("split_soup_count"); return -1; }
+    if (cudaMemsetAsync(w.total, 0, 16, st) != cudaSuccess ||
+        (hist.bins && cudaMemsetAsync(hist.bins, 0, kSplitBins * sizeof(int), st) != cudaSuccess)) {
+        *rc = check_launch("split_soup_count");
+        return -1;
+    }
     if (M > 0) {
         split_top_kernel<false><<<blocks_for(M, kSplitThreads), kSplitThreads, 0, st>>>(
             P, nullptr, plan, 0, M, verts, faces, valid, quota, w.table, w.top_count, nullptr, nullptr, nullptr,
-            nullptr, nullptr, w.probe_status, w.total, SplitHist{});
+            nullptr, nullptr, w.probe_status, w.total, hist);
         split_task_kernel<false><<<blocks_for((int64_t)M * kTopNodes, kSplitThreads), kSplitThreads, 0, st>>>(
             P, nullptr, plan, 0, M, verts, faces, w.table, w.top_count, w.task_counts, nullptr, nullptr, nullptr,
-            nullptr, nullptr, nullptr, w.probe_status, w.total, SplitHist{});
+            nullptr, nullptr, nullptr, w.probe_status, w.total, hist);
         if ((*rc = device_scan<int, int>(w.task_counts, (int64_t)M * kTopNodes, w.task_scan, true, w.scan_tasks, st)))
             return -1;
         split_family_kernel<<<blocks_for(M, kSplitThreads), kSplitThreads, 0, st>>>(M, w.top_count, w.task_scan,
                                                                                      w.counts, w.probe_status);
     }
     int64_t* total_dev = nullptr;
-    if ((*rc = device_scan<int, int64_t>(w.counts, M, offsets, false, w.scan, st, &total_dev))) return -1;
+    if ((*rc = device_scan<int, int64_t>(w.counts, M, offsets, false, w.scan, st, &total_dev, offsets + M))) return -1;
     int64_t total = 0;
     int pst = 0;
-    if (cudaMemcpyAsync(offsets + M, total_dev, sizeof(int64_t), cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(&total, total_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    if (cudaMemcpyAsync(&total, total_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(&pst, w.probe_status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        (hist.bins && cudaMemcpyAsync(bins_host, hist.bins, kSplitBins * sizeof(int), cudaMemcpyDeviceToHost, st) !=
+                          cudaSuccess) ||
         cudaStreamSynchronize(st) != cudaSuccess) {
         *rc = check_launch("split_soup_count");
         return -1;
@@ -565,16 +581,13 @@ static int64_t count_pass(const SplitParams& P, SplitPlan plan, const int* quota
     return (pst & DS_STATUS_SPLIT_LIMIT) ? -1 : total;
 }
 
-static float bits_float(unsigned b);
-
 // One pass of the budget's search: the splits of key >= lo (bits) are walked and
 // those of key < hi counted into bins of the bits (*shift receives the bins'
 // width).  Returns their number, or -1 when the walk met the limits.  One
 // read-back per pass, and neither per-face counts nor scans.
 static int64_t search_pass(const SplitParams& P, unsigned lo, unsigned hi, int M, const float* verts, const int* faces,
                            const int* valid, const SplitWs& w, cudaStream_t st, int* bins, int* shift, int* rc) {
-    SplitHist h{w.hist, lo, hi, 0};
-    while (((hi - lo - 1) >> h.shift) >= (unsigned)kSplitBins) ++h.shift;
+    const SplitHist h = split_bins(w.hist, lo, hi);
     const int used = (int)((hi - lo - 1) >> h.shift) + 1;
     *shift = h.shift;
     *rc = DS_OK;
@@ -601,9 +614,6 @@ static int64_t search_pass(const SplitParams& P, unsigned lo, unsigned hi, int M
     for (int i = 0; i < used; ++i) n += bins[i] = got[i];
     return (got[kSplitBins] & DS_STATUS_SPLIT_LIMIT) || n > kMaxTotalSplits ? -1 : n;
 }
-
-static float bits_float(unsigned b) { float f; std::memcpy(&f, &b, 4); return f; }
-static unsigned float_bits(float f) { unsigned b; std::memcpy(&b, &f, 4); return b; }
 
 }  // namespace dsb
 
@@ -649,32 +659,40 @@ int ds_split_soup_count(int mode, const float* mvp_host, float aspect_wh, float 
         // Search the squared length lam with count(lam) <= K < count(prev(lam)); the R = K - count(lam) missing
         // splits are edges of exactly prev(lam), taken in face order (the reference's heap takes such ties in
         // an unspecified order).
+        // Every pass counts the keys below `ok` in 2048 bins of their bits, so the pass that finds a `bad`
+        // (count above K) also says which bin holds the cut-off, and two more passes end what a bisection of the
+        // 2^23 lengths of an octave took 23 for (resampling 15,000 faces under a cap of 1,000 splits:
+        // 3.2 -> 1.1 ms, visibility counting included).
         const int64_t K = num_splits;
-        if (tau > 0.f) {
-            total = count_pass(P, SplitPlan{tau2, 0.f}, nullptr, M, verts, faces, vmask, split_offsets, w, st, &rc);
+        unsigned ok = 0x7f800001u, bad = 0;  // count(ok) = n_ok <= K (nothing above infinity), count(bad) > K
+        int64_t n_ok = 0;
+        int bins[kSplitBins], shift = 0;
+        bool have_bad = false, binned = false;  // binned: the bins are those of [bad, ok)
+        if (tau > 0.f) {  // the threshold's own count, with the bins of all keys above it
+            const SplitHist h = split_bins(w.hist, float_bits(tau2), ok);
+            total = tau2 < INFINITY ? count_pass(P, SplitPlan{tau2, 0.f}, nullptr, M, verts, faces, vmask, split_offsets,
+                                                 w, st, &rc, h, bins)
+                                    : 0;
             if (rc) return rc;
             if (total >= 0 && total <= K) plan = SplitPlan{tau2, 0.f};
+            else if (total >= 0) { bad = h.lo; shift = h.shift; have_bad = binned = true; }
         }
         if (!(plan.tau2 < INFINITY)) {
-            DS_CUDA(cudaMemsetAsync(w.max_bits, 0, sizeof(unsigned), st));
-            split_max_edge_kernel<<<blocks_for(M, kSplitThreads), kSplitThreads, 0, st>>>(P, M, verts, faces, vmask,
-                                                                                        w.max_bits);
-            unsigned hi_bits = 0;
-            DS_CUDA(cudaMemcpyAsync(&hi_bits, w.max_bits, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-            DS_CUDA(cudaStreamSynchronize(st));
+            unsigned hi_bits = ok - 1;
             const unsigned floor_bits = tau > 0.f ? float_bits(tau2) : 1u;  // lam stays >= tau^2 (> 0)
+            if (!have_bad) {
+                DS_CUDA(cudaMemsetAsync(w.max_bits, 0, sizeof(unsigned), st));
+                split_max_edge_kernel<<<blocks_for(M, kSplitThreads), kSplitThreads, 0, st>>>(P, M, verts, faces, vmask,
+                                                                                            w.max_bits);
+                DS_CUDA(cudaMemcpyAsync(&hi_bits, w.max_bits, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+                DS_CUDA(cudaStreamSynchronize(st));
+                ok = hi_bits + 1;
+            }
             if (hi_bits == 0 || hi_bits < floor_bits) {
                 total = 0;  // nothing reaches the threshold
             } else {
-                // count(hi) <= K is not certain (equal longest edges): walk down until count > K or the floor.
-                // Every pass counts the keys below `ok` in 2048 bins of their bits, so the pass that finds
-                // `bad` also says which bin holds the cut-off, and two passes end what a bisection of the
-                // 2^23 lengths of an octave took 23 for (resampling 15,000 faces under a cap of 1,000 splits:
-                // 3.3 -> 1.4 ms, visibility counting included).
-                unsigned ok = hi_bits + 1, bad = 0;  // count(ok) = n_ok <= K, count(bad) > K
-                int64_t n_ok = 0;
-                int bins[kSplitBins], shift = 0;
-                bool have_bad = false, binned = false;  // binned: the bins are those of [bad, ok)
+                // without a threshold (or where its tree met the limits): count(hi) <= K is not certain (equal
+                // longest edges), so walk down until count > K or the floor
                 unsigned probe = hi_bits;
                 for (int it = 0; it < 64 && !have_bad; ++it) {
                     const int64_t c = search_pass(P, probe, ok, M, verts, faces, vmask, w, st, bins, &shift, &rc);
