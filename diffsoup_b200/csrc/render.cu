@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(kThreads) deferred_shade_kernel(
     float* __restrict__ rgb, uchar4* __restrict__ rgba8) {
     __shared__ RenderWeights w;
     __shared__ __align__(16) float act_all[kRenderWarps][32 * kActStride];
+    chain_wait();
     // params: W1 [16,16], b1 [16], W2 [16,16], b2 [16], W3 [3,16], b3 [3]
     for (int i = threadIdx.x; i < 40 * kActStride; i += blockDim.x) {
         const int n = i / kActStride, k = i - n * kActStride;
@@ -288,10 +289,10 @@ static int launch_post(int B, const ds_view_desc* views, int64_t num_pixels, con
                        const float* inv_mvp, const float* mlp_params, float bg_r, float bg_g, float bg_b, float* rgb,
                        unsigned char* rgba8, cudaStream_t st) {
     if (num_pixels == 0) return DS_OK;
-    deferred_shade_kernel<<<pixel_grid(num_pixels), kThreads, 0, st>>>(
-        B, views, num_pixels, reinterpret_cast<const float4*>(gbuf), level, (int)feats_at_level((uint32_t)level),
-        reinterpret_cast<const uchar4*>(lut0), reinterpret_cast<const uchar4*>(lut1), num_texels, inv_mvp,
-        mlp_params, bg_r, bg_g, bg_b, rgb, reinterpret_cast<uchar4*>(rgba8));
+    launch_chained(deferred_shade_kernel, dim3(pixel_grid(num_pixels)), kThreads, 0, st, B, views, num_pixels,
+                   reinterpret_cast<const float4*>(gbuf), level, (int)feats_at_level((uint32_t)level),
+                   reinterpret_cast<const uchar4*>(lut0), reinterpret_cast<const uchar4*>(lut1), num_texels, inv_mvp,
+                   mlp_params, bg_r, bg_g, bg_b, rgb, reinterpret_cast<uchar4*>(rgba8));
     return check_launch("render_deferred");
 }
 

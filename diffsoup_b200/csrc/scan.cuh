@@ -46,6 +46,7 @@ __device__ __forceinline__ int64_t block_exclusive_scan(int64_t v, int64_t& excl
 template <typename In>
 __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const In* __restrict__ in, int64_t n,
                                                                         int64_t* __restrict__ partials) {
+    chain_wait();
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int64_t s = 0;
 #pragma unroll
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_block_sums_kernel(const In*
 // null) receives the total.
 static __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(int64_t* __restrict__ partials, int64_t nb,
                                                                             int64_t* __restrict__ total) {
+    chain_wait();
     int64_t carry = 0;
     for (int64_t start = 0; start < nb; start += kScanThreads) {
         const int64_t i = start + threadIdx.x;
@@ -79,6 +81,7 @@ template <typename In, typename Out>
 __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const In* __restrict__ in, int64_t n,
                                                                    const int64_t* __restrict__ partials,
                                                                    Out* __restrict__ out, bool inclusive) {
+    chain_wait();
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int64_t v[kScanItems];
     int64_t s = 0;
@@ -112,9 +115,9 @@ int device_scan(const In* in, int64_t n, Out* out, bool inclusive, void* ws, cud
         if (total_copy) DS_CUDA(cudaMemsetAsync(total_copy, 0, sizeof(int64_t), st));
         return DS_OK;
     }
-    scan_block_sums_kernel<In><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, partials);
-    scan_partials_kernel<<<1, kScanThreads, 0, st>>>(partials, nb, total_copy);
-    scan_apply_kernel<In, Out><<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, partials, out, inclusive);
+    launch_chained(scan_block_sums_kernel<In>, dim3((unsigned)nb), kScanThreads, 0, st, in, n, partials);
+    launch_chained(scan_partials_kernel, dim3(1), kScanThreads, 0, st, partials, nb, total_copy);
+    launch_chained(scan_apply_kernel<In, Out>, dim3((unsigned)nb), kScanThreads, 0, st, in, n, partials, out, inclusive);
     return check_launch("device_scan");
 }
 
@@ -130,6 +133,7 @@ constexpr int64_t kScanOneMax = (int64_t)kScanOneThreads * kScanOneItems;
 // out[i] = sum of in[0..i) for i < n and out[n] = the total (n <= kScanOneMax).
 static __global__ void __launch_bounds__(kScanOneThreads) scan_one_cta_kernel(const int* __restrict__ in, int n,
                                                                               int64_t* __restrict__ out) {
+    chain_wait();
     __shared__ int64_t warp_tot[kScanOneThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int per = (n + kScanOneThreads - 1) / kScanOneThreads;  // <= kScanOneItems

@@ -166,6 +166,7 @@ __device__ __forceinline__ float2 relu_gate(const __nv_bfloat16* h, float2 v) {
 
 template <class K>
 __global__ void __launch_bounds__(K::WARPS * 32, K::REG_GRADS ? DSB_SHADE_MIN_CTAS : 1) shade_step_kernel(ShadeArgs a) {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ShadeSmem<K>& sm = *reinterpret_cast<ShadeSmem<K>*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

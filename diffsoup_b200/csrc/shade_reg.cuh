@@ -161,6 +161,7 @@ __device__ __forceinline__ void reg_weights(RegWeights<K>& f, const float* __res
 
 template <class K>
 __global__ void __launch_bounds__(kShadeRegWarps * 32, K::MIN_CTAS) shade_reg_kernel(ShadeArgs a) {
+    chain_wait();
     constexpr int NS = K::NS, IN = K::IN, C = K::C, NL = K::NL;
     extern __shared__ __align__(16) unsigned char reg_smem_raw[];  // RegSmem<K> (above the 48 KB static limit)
     RegSmem<K>& sm = *reinterpret_cast<RegSmem<K>*>(reg_smem_raw);

@@ -136,6 +136,7 @@ struct __align__(1024) TcSmem {
 };
 
 __global__ void __launch_bounds__(kTcThreads, 2) shade_tc_kernel(ShadeArgs a) {
+    chain_wait();
     using K = ShadeCfg<16, 32, 64, 2>;
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     TcSmem& sm = *reinterpret_cast<TcSmem*>(tc_smem_raw);

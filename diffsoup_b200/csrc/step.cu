@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(kMapWarps * 32) accum_tab_backward_kernel(
     float* __restrict__ feat_src_grad, const int2* __restrict__ adj_ent, const int* __restrict__ adj_row) {
     constexpr int G = kTabGroup<CP>, GW = kTabGroupWarps<CP>, L = 32 * GW, Q = CP / 4;
     extern __shared__ __align__(16) unsigned char map_smem[];
+    chain_wait();
     const int N = ST * (hi - lo + 1) * 3;
     MapRows m;
     m.ent = reinterpret_cast<int2*>(map_smem);
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(kEdgeThreads, DSB_EDGE_MIN_CTAS) edge_step_ker
     const float* __restrict__ color, const float* __restrict__ grad_color, const float* __restrict__ rast,
     double* __restrict__ grad_pos) {
     __shared__ EdgeHalo h;
+    chain_wait();
     const int tile = blockIdx.x;
     // no triangle may cover a pixel centre of the tile (its list is empty): every pixel is background,
     // and background pixels contribute nothing as the centre of a pair
@@ -557,7 +559,7 @@ static int launch_shade(const ShadeArgs& a, cudaStream_t st) {
     const int64_t want = (chunks + K::WARPS - 1) / K::WARPS;
     const int64_t cap = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);
     const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-    shade_step_kernel<K><<<grid, K::WARPS * 32, smem, st>>>(a);
+    launch_chained(shade_step_kernel<K>, dim3(grid), K::WARPS * 32, smem, st, a);
     return check_launch("shade_step");
 }
 
@@ -575,7 +577,7 @@ static int launch_shade_reg(const ShadeArgs& a, cudaStream_t st) {
     const int64_t want = (chunks + kShadeRegWarps - 1) / kShadeRegWarps;
     const int64_t cap = (int64_t)sm_count() * per_sm;
     const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-    shade_reg_kernel<K><<<grid, kShadeRegWarps * 32, smem, st>>>(a);
+    launch_chained(shade_reg_kernel<K>, dim3(grid), kShadeRegWarps * 32, smem, st, a);
     return check_launch("shade_reg");
 }
 
@@ -608,7 +610,7 @@ static int launch_shade_tc(const ShadeArgs& a, cudaStream_t st) {
     const int64_t tiles = (a.num_pixels + kTcThreads - 1) / kTcThreads;
     const int64_t cap = (int64_t)sm_count() * per_sm;
     const unsigned grid = (unsigned)(tiles < 1 ? 1 : (tiles < cap ? tiles : cap));
-    shade_tc_kernel<<<grid, kTcThreads, smem, st>>>(a);
+    launch_chained(shade_tc_kernel, dim3(grid), kTcThreads, smem, st, a);
     return check_launch("shade_tc");
 }
 
@@ -880,8 +882,13 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
         const int per = kTabGroup<CPP> * (kMapWarps / kTabGroupWarps<CPP>); /* triangles of a CTA's pass */        \
         const int64_t want = ((int64_t)c.T + per - 1) / per;                                                       \
         const int64_t wave = (int64_t)sm_count() * per_sm - EXTRA;                                                 \
-        KERNEL<CC, CPP><<<(unsigned)((want < wave ? want : wave) + EXTRA), kMapWarps * 32, tsm, STREAM>>>(         \
-            c.T, c.min_level, c.max_level, S, ST, __VA_ARGS__);                                                    \
+        const dim3 tgrid((unsigned)((want < wave ? want : wave) + EXTRA));                                         \
+        if (BWD) /* after the opacity pass; the forward follows an event wait */                                   \
+            launch_chained(KERNEL<CC, CPP>, tgrid, kMapWarps * 32, tsm, STREAM, c.T, c.min_level, c.max_level, S, ST, \
+                           __VA_ARGS__);                                                                           \
+        else                                                                                                       \
+            KERNEL<CC, CPP><<<tgrid, kMapWarps * 32, tsm, STREAM>>>(c.T, c.min_level, c.max_level, S, ST,          \
+                                                                    __VA_ARGS__);                                  \
     } while (0)
 #define DSB_TAB_C(KERNEL, BWD, EXTRA, STREAM, ...)                                                                 \
     do {                                                                                                           \
@@ -910,7 +917,7 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
     if (rc || (rc = mark(2, st))) return rc;
     if (side && (rc = join_from(side, 0, st))) return rc;  // the rasterizer reads the accumulated opacities
     rc = tiles_rasterize_impl(c.B, views, num_tiles, c.T, c.max_level, ST, w.alpha_acc, c.stochastic ? 1 : 0,
-                              c.thr_const, rng, rast, w.tiles, list_capacity, rs, st, block_shape_log2(c));
+                              c.thr_const, rng, rast, w.tiles, list_capacity, rs, st, block_shape_log2(c), side == nullptr);
     if (rc || (rc = mark(3, st))) return rc;
 
     // fused shading forward + backward
@@ -967,9 +974,9 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
     if ((rc = mark(5, st))) return rc;
 
     // edge gradients to clip-space positions
-    edge_step_kernel<<<(unsigned)num_tiles, kEdgeThreads, 0, st>>>(
-        c.B, views, c.V, c.T, tiles_tables(w.tiles, c.B, c.T, num_tiles, list_capacity), tri, a.color, w.grad_color,
-        rast, w.grad_pos);
+    launch_chained(edge_step_kernel, dim3((unsigned)num_tiles), kEdgeThreads, 0, st, c.B, views, c.V, c.T,
+                   tiles_tables(w.tiles, c.B, c.T, num_tiles, list_capacity), tri, a.color, w.grad_color, rast,
+                   w.grad_pos);
     if ((rc = mark(6, st))) return rc;
     if (side && (rc = join_from(side, 1, st))) return rc;
     // (one stream: the phases in order, so that the profiling events time each alone)

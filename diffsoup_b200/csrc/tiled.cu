@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(kThreads) bin_setup_kernel(int B, const ds_vie
                                                              TriVerts* __restrict__ verts, TriNdc* __restrict__ ndc,
                                                              TriEdges* __restrict__ edges, int* __restrict__ counts) {
     __shared__ unsigned long long s_mask[kThreads];
+    chain_wait();
     const int64_t i = bin_record<TPW>((int64_t)B * T);
     const bool live = i < (int64_t)B * T;
     const int b = live ? (int)(i / T) : 0, t = live ? (int)(i % T) : 0;
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(kThreads) bin_fill_kernel(int B, const ds_view
                                                             const int64_t* __restrict__ offsets,
                                                             int* __restrict__ cursor, ListEntry* __restrict__ list,
                                                             int64_t capacity, int* __restrict__ status) {
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int64_t i = bin_record<TPW>((int64_t)B * T);
     const bool live = i < (int64_t)B * T;
@@ -439,6 +441,7 @@ __global__ void __launch_bounds__(kSortWarps * 32) sort_lists_kernel(int num_til
                                                                      const ListEntry* __restrict__ fill,
                                                                      ListEntry* __restrict__ list, int64_t capacity,
                                                                      int* __restrict__ sorted) {
+    chain_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x * kSortWarps + warp;
     if (tile >= num_tiles) return;
@@ -711,6 +714,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RasterStage& st = s_stage[warp];
     WarpRecs& R = s_rec[REC ? warp : 0];
+    chain_wait();
     uint64_t seed = 0;
     uint32_t iter = 0;
     if (thr_mode == 1) { seed = rng[0]; iter = (uint32_t)rng[1]; }
@@ -898,6 +902,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
     __shared__ RasterStage s_stage[kWarpsPerCta];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RasterStage& st = s_stage[warp];
+    chain_wait();
     const int items = item_list ? *item_count : num_tiles * kBlocksPerTile;
     for (int n = warp_next(work, items); n < items; n = warp_next(work, items)) {
         const int item = item_list ? item_list[n] : n;
@@ -983,11 +988,12 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
     const unsigned grid = blocks_for(narrow ? n * 4 : n);  // 8 or 32 triangles per warp
     if (n > 0) {
         const auto setup = narrow ? bin_setup_kernel<8> : bin_setup_kernel<32>;
-        setup<<<grid, kThreads, 0, st>>>(B, views, V, pos, T, tri, w.boxes, w.verts, w.ndc, w.edges, w.counts);
+        launch_chained(setup, dim3(grid), kThreads, 0, st, B, views, V, pos, T, tri, w.boxes, w.verts, w.ndc, w.edges,
+                       w.counts);
     }
     // offsets[num_tiles] = total number of entries; up to kScanOneMax tiles in one launch
     if (num_tiles <= kScanOneMax) {
-        scan_one_cta_kernel<<<1, kScanOneThreads, 0, st>>>(w.counts, num_tiles, w.offsets);
+        launch_chained(scan_one_cta_kernel, dim3(1), kScanOneThreads, 0, st, w.counts, num_tiles, w.offsets);
     } else {
         rc = device_scan<int, int64_t>(w.counts, num_tiles, w.offsets, false, w.scan, st, nullptr,
                                        w.offsets + num_tiles);
@@ -995,12 +1001,12 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
     }
     if (n > 0) {
         const auto fill = narrow ? bin_fill_kernel<8> : bin_fill_kernel<32>;
-        fill<<<grid, kThreads, 0, st>>>(B, views, T, w.boxes, w.verts, w.ndc, w.offsets, w.cursor, w.fill,
-                                        list_capacity, status);
+        launch_chained(fill, dim3(grid), kThreads, 0, st, B, views, T, w.boxes, w.verts, w.ndc, w.offsets, w.cursor,
+                       w.fill, list_capacity, status);
     }
     if (num_tiles > 0)
-        sort_lists_kernel<<<(unsigned)((num_tiles + kSortWarps - 1) / kSortWarps), kSortWarps * 32, 0, st>>>(
-            num_tiles, w.offsets, w.fill, w.list, list_capacity, w.sorted);
+        launch_chained(sort_lists_kernel, dim3((unsigned)((num_tiles + kSortWarps - 1) / kSortWarps)), kSortWarps * 32, 0,
+                       st, num_tiles, w.offsets, w.fill, w.list, list_capacity, w.sorted);
     return check_launch("tiles_bin");
 }
 
@@ -1046,19 +1052,32 @@ static int g_occ_raster = 0, g_occ_raster_rec = 0, g_occ_aux = 0;
 
 int tiles_rasterize_impl(int B, const ds_view_desc* views, int num_tiles, int T, int level, int S,
                          const float* alpha_src, int thr_mode, float thr_const, const uint64_t* rng, float* rast,
-                         void* workspace, int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl) {
+                         void* workspace, int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl,
+                         bool chained) {
     if (num_tiles == 0) return DS_OK;
     TileWs w = carve(workspace, B, T, num_tiles, list_capacity, nullptr);
     if (rs != nullptr) {
         const void* k = reinterpret_cast<const void*>(&raster_kernel<true>);
-        raster_kernel<true><<<block_grid(num_tiles, k, g_occ_raster_rec), kWarpsPerCta * 32, 0, st>>>(
-            B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
-            alpha_src, thr_mode, thr_const, rng, w.work, rast, *rs, bwl);
+        const dim3 grid(block_grid(num_tiles, k, g_occ_raster_rec));
+        if (chained)
+            launch_chained(raster_kernel<true>, grid, kWarpsPerCta * 32, 0, st, B, views, num_tiles, T, w.boxes, w.verts,
+                           w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, thr_mode, thr_const,
+                           rng, w.work, rast, *rs, bwl);
+        else
+            raster_kernel<true><<<grid, kWarpsPerCta * 32, 0, st>>>(
+                B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
+                alpha_src, thr_mode, thr_const, rng, w.work, rast, *rs, bwl);
     } else {
         const void* k = reinterpret_cast<const void*>(&raster_kernel<false>);
-        raster_kernel<false><<<block_grid(num_tiles, k, g_occ_raster), kWarpsPerCta * 32, 0, st>>>(
-            B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
-            alpha_src, thr_mode, thr_const, rng, w.work, rast, RecordStore{}, bwl);
+        const dim3 grid(block_grid(num_tiles, k, g_occ_raster));
+        if (chained)
+            launch_chained(raster_kernel<false>, grid, kWarpsPerCta * 32, 0, st, B, views, num_tiles, T, w.boxes, w.verts,
+                           w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, thr_mode, thr_const,
+                           rng, w.work, rast, RecordStore{}, bwl);
+        else
+            raster_kernel<false><<<grid, kWarpsPerCta * 32, 0, st>>>(
+                B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
+                alpha_src, thr_mode, thr_const, rng, w.work, rast, RecordStore{}, bwl);
     }
     return check_launch("tiles_rasterize");
 }
@@ -1069,10 +1088,9 @@ static int aux_launch(int B, const ds_view_desc* views, int num_tiles, int T, in
                       const int* item_list, const int* item_count, cudaStream_t st, int bwl) {
     TileWs w = carve(workspace, B, T, num_tiles, list_capacity, nullptr);
     const void* k = reinterpret_cast<const void*>(&aux_kernel);
-    aux_kernel<<<block_grid(num_tiles, k, g_occ_aux), kWarpsPerCta * 32, 0, st>>>(
-        B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
-        alpha_src, C,
-        color, target, rast, scale, item_list, item_count, w.work + 1, grad_alpha_src, bwl);
+    launch_chained(aux_kernel, dim3(block_grid(num_tiles, k, g_occ_aux)), kWarpsPerCta * 32, 0, st, B, views, num_tiles, T,
+                   w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, C, color,
+                   target, rast, scale, item_list, item_count, w.work + 1, grad_alpha_src, bwl);
     return check_launch("tiles_opacity_aux");
 }
 
@@ -1110,7 +1128,7 @@ int ds_tiles_rasterize(int B, const ds_view_desc* views, int num_tiles, int V, c
     DS_CHECK_ARG(thr_mode == 0 || (thr_mode == 1 && rng != nullptr), "tiles_rasterize: bad threshold mode");
     DS_CHECK_ARG(((uintptr_t)rast & 15) == 0, "tiles_rasterize: rast not 16-byte aligned");
     return tiles_rasterize_impl(B, views, num_tiles, T, level, S, alpha_src, thr_mode, thr_const, rng, rast,
-                                workspace, list_capacity, nullptr, (cudaStream_t)stream, kDefaultBlockShape);
+                                workspace, list_capacity, nullptr, (cudaStream_t)stream, kDefaultBlockShape, true);
 }
 
 int ds_tiles_opacity_aux(int B, const ds_view_desc* views, int num_tiles, int V, const float* pos, int T,
