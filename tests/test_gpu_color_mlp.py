@@ -14,12 +14,19 @@ DEV = "cuda"
 
 def make(cin, layers, shape, cover, seed=0):
     g = torch.Generator(device=DEV).manual_seed(seed)
+    torch.manual_seed(seed)
     mlp = ColorMLP(cin, 3, 16, layers).to(DEV)
     with torch.no_grad():
         for p in mlp.parameters():
             p.add_(0.1 * torch.randn(p.shape, generator=g, device=DEV))
     x = torch.rand(*shape, cin, generator=g, device=DEV)
     mask = None if cover is None else torch.rand(*shape, generator=g, device=DEV) < cover
+    if mask is not None:  # a pixel whose hidden sum is zero within FP32 rounding has no FP64 gradient to compare with
+        h = x.double()
+        for lin in [m for m in mlp.mlp if isinstance(m, torch.nn.Linear)][:-1]:
+            z = h @ lin.weight.double().T + lin.bias.double()
+            mask &= (z.abs() > 1e-5).all(-1)
+            h = torch.relu(z)
     return mlp, x, mask, torch.randn(*shape, 3, generator=g, device=DEV)
 
 
@@ -36,8 +43,6 @@ def run(mlp, x, mask, gout):
 @pytest.mark.parametrize("shape,cover", [((1, 1, 1), None), ((1, 3, 11), 0.5), ((2, 16, 17), 0.02), ((1, 401, 397), 0.6)])
 def test_matches_torch_in_fp64(cin, layers, shape, cover):
     mlp, x, mask, g = make(cin, layers, shape, cover, seed=cin)
-    if mask is not None:
-        mask.view(-1)[-1] = True
     assert mlp._fused_layers(x, mask) is not None
     got = run(mlp, x, mask, g)
     d = copy.deepcopy(mlp).double()
