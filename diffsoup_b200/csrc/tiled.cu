@@ -825,9 +825,9 @@ __device__ __forceinline__ void aux_scatter(float b0, float b1, int level, int S
 }
 
 // Opacity auxiliary gradient from the fragment records: one thread per
-// record, blocks stride over the chunks.  A chunk holds whole 8x4 blocks in
-// walk order, so neighbouring records often share a triangle and a lattice
-// cell: runs of equal (triangle, cell) in a warp are summed with a segmented
+// record, blocks stride over the chunks.  Records follow the rasterizer's
+// passes, so neighbours that share a triangle and a lattice cell come from
+// neighbouring pixels of one pass: runs of equal (triangle, cell) in a warp are summed with a segmented
 // reduction before the global atomics.
 __global__ void __launch_bounds__(kRecChunk) aux_records_kernel(RecordStore rs, int level, int S,
                                                                const float* __restrict__ alpha_src,
