@@ -83,14 +83,17 @@ def rasterize_multires_triangle_alpha(resolution: Tuple[int, int], pos: torch.Te
 # ---------------------------------------------------------------------------
 
 def _shade(x: torch.Tensor, mask: Optional[torch.Tensor], weights, biases: torch.Tensor) -> torch.Tensor:
-    """The fused kernels' function of flat rows x [n,in], in torch operations (their double backward)."""
+    """The fused kernels' function of flat rows x [n,in], in torch operations (their double backward).  Only the
+    rows that mask covers are computed, as the kernels do: an infinity or NaN of another row would turn its zero
+    gradient into NaN."""
+    if mask is not None:
+        return torch.zeros_like(x[:, :3]).index_put((mask,), _shade(x[mask], None, weights, biases))
     h, o = x, 0
     for w in weights:
         h = nn.functional.linear(h, w, biases[o:o + w.shape[0]])
         o += w.shape[0]
         h = torch.sigmoid(h) if w is weights[-1] else torch.relu(h)
-    y = (1.0 - x[:, 3:4]) * x[:, :3] + x[:, 3:4] * h
-    return y if mask is None else torch.where(mask.unsqueeze(-1), y, torch.zeros_like(y))
+    return (1.0 - x[:, 3:4]) * x[:, :3] + x[:, 3:4] * h
 
 
 class _ColorMLPFn(torch.autograd.Function):

@@ -1,0 +1,63 @@
+"""ColorMLP's torch form of the fused kernels, which a differentiable backward goes through: values of pixels that the
+mask leaves out reach no gradient."""
+
+import types
+
+import pytest
+import torch
+
+from diffsoup_b200 import ColorMLP, multires
+
+
+def rows(dev, n=60, cin=11):
+    g = torch.Generator().manual_seed(3)
+    torch.manual_seed(3)
+    mlp = ColorMLP(cin, 3, 16, 2).to(dev)
+    x, mask = torch.rand(1, 1, n, cin, generator=g), torch.rand(1, 1, n, generator=g) < 0.6
+    mask[0, 0, :3] = False
+    clean = x.clone()
+    x[0, 0, 0], x[0, 0, 1, 5], x[0, 0, 2, 3] = float("nan"), float("inf"), float("-inf")
+    return mlp, x.to(dev), clean.to(dev), mask.to(dev), torch.randn(1, 1, n, 3, generator=g).to(dev)
+
+
+def backward_on(mlp, x, mask, g):
+    """_ColorMLPFn.backward with gradients enabled, as create_graph runs it: gradients of x, biases and weights."""
+    lins = [m for m in mlp.mlp if isinstance(m, torch.nn.Linear)]
+    saved = (x.view(-1, x.shape[-1]), None if mask is None else mask.view(-1), torch.cat([m.bias for m in lins]),
+             *[m.weight for m in lins])
+    ctx = types.SimpleNamespace(saved_tensors=saved, needs_input_grad=[True, False] + [True] * (len(lins) + 1))
+    gx, _, gb, *gw = multires._ColorMLPFn.backward(ctx, g.view(-1, 3))
+    return [gx.view_as(x), gb, *gw]
+
+
+def test_differentiable_backward_leaves_masked_rows_out():
+    """First gradients with create_graph, and a second derivative, against the module on rows without infinities and
+    NaN."""
+    mlp, x, clean, mask, g = rows("cpu")
+    lins = [m for m in mlp.mlp if isinstance(m, torch.nn.Linear)]
+    weights = [m.weight for m in lins]
+
+    def second(first):
+        return torch.autograd.grad(first[0][mask].square().sum() + first[2].square().sum(), weights)
+
+    x.requires_grad_(True)
+    got = backward_on(mlp, x, mask, g)
+    clean.requires_grad_(True)
+    want = torch.autograd.grad(mlp(clean, mask=mask), [clean, *[m.bias for m in lins], *weights], g, create_graph=True)
+    want = [want[0], torch.cat(want[1:4]), *want[4:]]
+    for a, b in zip([*got, *second(got)], [*want, *second(want)]):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.gpu
+def test_create_graph_leaves_masked_rows_out():
+    """The call with create_graph=True, on the rows with infinities and NaN, against the clean rows without it."""
+    mlp, x, clean, mask, g = rows("cuda")
+    assert mlp._fused_layers(x, mask) is not None
+
+    def grads(x, create_graph):
+        x = x.clone().requires_grad_(True)
+        return torch.autograd.grad(mlp(x, mask=mask), [x, *mlp.parameters()], g, create_graph=create_graph)
+
+    for a, b in zip(grads(x, True), grads(clean, False)):
+        torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
