@@ -82,18 +82,34 @@ def rasterize_multires_triangle_alpha(resolution: Tuple[int, int], pos: torch.Te
 #  Colour MLP (multires.py:109-207)
 # ---------------------------------------------------------------------------
 
-def _shade(x: torch.Tensor, mask: Optional[torch.Tensor], weights, biases: torch.Tensor) -> torch.Tensor:
-    """The fused kernels' function of flat rows x [n,in], in torch operations (their double backward).  Only the
-    rows that mask covers are computed, as the kernels do: an infinity or NaN of another row would turn its zero
-    gradient into NaN."""
+def _gradients(x: torch.Tensor, mask: Optional[torch.Tensor], biases: torch.Tensor, weights, grad_out: torch.Tensor,
+               need_x: bool):
+    """The backward kernels' gradients of flat rows x [n,in] (None unless need_x), biases and weights in torch
+    operations, which are differentiable.  Only the rows that mask covers are computed, as the kernels do: an
+    infinity or NaN of another row would turn its zero gradient into NaN."""
+    xs, g = x, grad_out
     if mask is not None:
-        return torch.zeros_like(x[:, :3]).index_put((mask,), _shade(x[mask], None, weights, biases))
-    h, o = x, 0
-    for w in weights:
-        h = nn.functional.linear(h, w, biases[o:o + w.shape[0]])
-        o += w.shape[0]
-        h = torch.sigmoid(h) if w is weights[-1] else torch.relu(h)
-    return (1.0 - x[:, 3:4]) * x[:, :3] + x[:, 3:4] * h
+        rows = mask.nonzero().squeeze(1)
+        xs, g = x.index_select(0, rows), grad_out.index_select(0, rows)
+    hs, b = [xs], biases.split([w.shape[0] for w in weights])
+    for w, bw in zip(weights[:-1], b):
+        hs.append(torch.relu(nn.functional.linear(hs[-1], w, bw)))
+    y = torch.sigmoid(nn.functional.linear(hs[-1], weights[-1], b[-1]))
+    res, aten = xs[:, 3:4], torch.ops.aten
+    d = aten.sigmoid_backward(res * g, y)
+    gw, gb = [], []
+    for i in range(len(weights) - 1, -1, -1):
+        gw.append(d.t() @ hs[i])
+        gb.append(d.sum(0))
+        if i > 0:
+            d = aten.threshold_backward(d @ weights[i], hs[i], 0.0)
+    gx = None
+    if need_x:
+        blend = torch.cat([(1.0 - res) * g, (g * (y - xs[:, :3])).sum(1, keepdim=True)], 1)
+        gx = d @ weights[0] + nn.functional.pad(blend, (0, x.shape[1] - 4))
+        if mask is not None:
+            gx = torch.zeros_like(x).index_copy(0, rows, gx)
+    return gx, torch.cat(gb[::-1]), gw[::-1]
 
 
 class _ColorMLPFn(torch.autograd.Function):
@@ -114,11 +130,8 @@ class _ColorMLPFn(torch.autograd.Function):
     def backward(ctx, grad_out):
         x, mask, biases, *weights = ctx.saved_tensors
         if torch.is_grad_enabled():  # create_graph: the gradient as differentiable operations
-            ins = [t for t, need in zip((x, biases, *weights), (ctx.needs_input_grad[0], *ctx.needs_input_grad[2:]))
-                   if need]
-            grads = iter(torch.autograd.grad(_shade(x, mask, weights, biases), ins, grad_out, create_graph=True))
-            need = ctx.needs_input_grad
-            return (next(grads) if need[0] else None, None, *(next(grads) if k else None for k in need[2:]))
+            gx, gb, gw = _gradients(x, mask, biases, weights, grad_out, ctx.needs_input_grad[0])
+            return (gx, None, gb, *gw)
         n, cin = x.shape
         layers = len(weights) - 1
         grad_out = grad_out.contiguous()

@@ -49,6 +49,29 @@ def test_differentiable_backward_leaves_masked_rows_out():
         torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("layers", [1, 2])
+@pytest.mark.parametrize("cover", [None, 0.0, 0.5, 1.0])
+def test_differentiable_backward_is_the_modules(layers, cover):
+    """Every gradient, and the gradients of a function of them, in FP64 (chains of at most 60 products and sums)."""
+    torch.manual_seed(layers)
+    mlp = ColorMLP(7, 3, 16, layers).double()
+    x = torch.randn(1, 6, 10, 7, dtype=torch.float64, requires_grad=True)
+    g = torch.randn(1, 6, 10, 3, dtype=torch.float64, requires_grad=True)
+    mask = None if cover is None else torch.rand(1, 6, 10) < cover
+    lins = [m for m in mlp.mlp if isinstance(m, torch.nn.Linear)]
+    weights, biases = [m.weight for m in lins], [m.bias for m in lins]
+    got = backward_on(mlp, x, mask, g)
+    y = mlp(x, mask=mask) + 0.0 * sum(t.sum() for t in (x, *weights, *biases))  # nothing covered: zero gradients
+    want = torch.autograd.grad(y, [x, *biases, *weights], g, create_graph=True)
+    want = [want[0], torch.cat(want[1:len(lins) + 1]), *want[len(lins) + 1:]]
+    for a, b in zip(got, want):
+        torch.testing.assert_close(a, b, rtol=1e-11, atol=1e-13)
+    second = [torch.autograd.grad(sum(t.sin().sum() for t in first), [x, g, *weights, *biases], materialize_grads=True)
+              for first in (got, want)]
+    for a, b in zip(*second):
+        torch.testing.assert_close(a, b, rtol=1e-10, atol=1e-12)
+
+
 @pytest.mark.gpu
 def test_create_graph_leaves_masked_rows_out():
     """The call with create_graph=True, on the rows with infinities and NaN, against the clean rows without it."""
