@@ -129,7 +129,8 @@ class _ColorMLPFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         x, mask, biases, *weights = ctx.saved_tensors
-        if torch.is_grad_enabled():  # create_graph: the gradient as differentiable operations
+        # create_graph, and a batch of gradients (vmap): the gradient in torch operations
+        if torch.is_grad_enabled() or not _plain_call(grad_out):
             gx, gb, gw = _gradients(x, mask, biases, weights, grad_out, ctx.needs_input_grad[0])
             return (gx, None, gb, *gw)
         n, cin = x.shape
@@ -149,10 +150,11 @@ class _ColorMLPFn(torch.autograd.Function):
 
 def _plain_call(*tensors) -> bool:
     """Whether nothing watches or transforms torch operations on these tensors (tracing, compilation, function
-    transforms, forward-mode AD, dispatch modes, autocast), so that a kernel may take their place."""
-    return (all(type(t) in (torch.Tensor, nn.Parameter) for t in tensors)
+    transforms, the batched gradients of autograd, forward-mode AD, dispatch modes), so that a kernel may take
+    their place."""
+    return (all(type(t) in (torch.Tensor, nn.Parameter) and not torch._C._functorch.is_legacy_batchedtensor(t)
+                for t in tensors)
             and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
-            and not torch.is_autocast_enabled("cuda")
             and torch._C._functorch.peek_interpreter_stack() is None
             and torch.autograd.forward_ad._current_level < 0
             and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
@@ -213,7 +215,7 @@ class ColorMLP(nn.Module):
                 or (mask is not None and not (type(mask) is torch.Tensor and mask.dtype == torch.bool
                                               and mask.device == x.device))
                 or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
-                or g._global_backward_pre_hooks or not all(_no_hooks(m) for m in mods + [self.mlp])):
+                or g._global_backward_pre_hooks or torch.is_autocast_enabled("cuda") or not all(_no_hooks(m) for m in mods + [self.mlp])):
             return None
         for lin, shape in zip(lins, shapes):
             if lin.bias is None or tuple(lin.weight.shape) != shape or any(

@@ -72,6 +72,59 @@ def test_differentiable_backward_is_the_modules(layers, cover):
         torch.testing.assert_close(a, b, rtol=1e-10, atol=1e-12)
 
 
+class TorchForward(torch.autograd.Function):
+    """_ColorMLPFn with the module's own operations in the forward, so that its backward runs without a GPU."""
+
+    @staticmethod
+    def forward(ctx, x, mask, biases, *weights):
+        ctx.save_for_backward(x, mask, biases, *weights)
+        mlp = ColorMLP(x.shape[1], 3, 16, len(weights) - 1)
+        with torch.no_grad():
+            for lin, w, b in zip([m for m in mlp.mlp if isinstance(m, torch.nn.Linear)], weights,
+                                 biases.split([w.shape[0] for w in weights])):
+                lin.weight.copy_(w), lin.bias.copy_(b)
+            return mlp(x[None, None], None if mask is None else mask[None, None])[0, 0]
+
+    backward = staticmethod(multires._ColorMLPFn.backward)
+
+
+def batched(out, inputs, gs):
+    """The three ways to ask for a batch of gradients, each against one gradient at a time."""
+    want = [torch.stack(t) for t in zip(*(torch.autograd.grad(out, inputs, g, retain_graph=True) for g in gs))]
+    one = lambda g: torch.autograd.grad(out, inputs, g, retain_graph=True)  # noqa: E731
+    for got in (torch.autograd.grad(out, inputs, gs, retain_graph=True, is_grads_batched=True),
+                torch.func.vmap(one)(gs),
+                torch.autograd.grad(out, inputs, gs, retain_graph=True, is_grads_batched=True, create_graph=True)):
+        for a, b in zip(got, want):
+            torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+def test_batched_gradients(masked):
+    mlp, _, x, mask, _ = rows("cpu")
+    lins = [m for m in mlp.mlp if isinstance(m, torch.nn.Linear)]
+    weights, x, mask = [m.weight for m in lins], x.view(-1, 11).requires_grad_(True), mask.view(-1) if masked else None
+    out = TorchForward.apply(x, mask, torch.cat([m.bias for m in lins]), *weights)
+    want = mlp(x[None, None], None if mask is None else mask[None, None])[0, 0]
+    gs = torch.randn(4, *out.shape, generator=torch.Generator().manual_seed(0))
+    inputs = [x, *mlp.parameters()]
+    for g in gs:  # backward without create_graph needs the kernels: compared through the batch of one
+        for a, b in zip(torch.autograd.grad(out, inputs, g[None], retain_graph=True, is_grads_batched=True),
+                        torch.autograd.grad(want, inputs, g, retain_graph=True)):
+            torch.testing.assert_close(a[0], b, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("masked", [False, True])
+def test_batched_gradients_of_the_fused_call(masked):
+    mlp, _, x, mask, _ = rows("cuda")
+    x.requires_grad_(True)
+    out = mlp(x, mask=mask if masked else None)
+    assert "_ColorMLPFn" in str(out.grad_fn.next_functions)
+    gs = torch.randn(4, *out.shape, generator=torch.Generator().manual_seed(0)).cuda()
+    batched(out, [x, *mlp.parameters()], gs)
+
+
 @pytest.mark.gpu
 def test_create_graph_leaves_masked_rows_out():
     """The call with create_graph=True, on the rows with infinities and NaN, against the clean rows without it."""
