@@ -73,6 +73,31 @@ int check_launch(const char* what);
             return ::dsb::set_error(DS_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
+constexpr int kSmemMax = 227 * 1024;  // dynamic shared memory of a CTA without static shared memory
+
+// CTAs of a kernel (the template argument: one record per kernel) that an SM of
+// the current device holds with `smem` bytes of dynamic shared memory, at least
+// 1.  The kernel's limit is a property of the device that all threads share, so it
+// is only ever set to kSmemMax: with each call's own size, a smaller call on
+// another thread could lower it between a call's setting and its launch.
+template <auto Kernel>
+inline int resident_ctas(int threads, size_t smem, int* per_sm) {
+    static thread_local int known_dev = -1, fit = 1;  // the thread's last answer
+    static thread_local size_t known_smem = 0;
+    int dev = 0;
+    DS_CUDA(cudaGetDevice(&dev));
+    if (dev != known_dev || smem != known_smem) {
+        known_dev = -1;
+        DS_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+        DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, Kernel, threads, smem));
+        if (fit < 1) fit = 1;
+        known_dev = dev;
+        known_smem = smem;
+    }
+    *per_sm = fit;
+    return DS_OK;
+}
+
 // View of a packed pixel index: the last view whose pix_offset <= p.
 __device__ __forceinline__ int view_of_pixel(const ds_view_desc* __restrict__ views, int B, int64_t p) {
     int lo = 0, hi = B - 1;

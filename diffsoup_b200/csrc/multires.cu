@@ -471,13 +471,13 @@ static size_t map_smem_bytes(int64_t T, int lo, int hi, int S, int ST, int C, bo
 template <int I, bool ADJOINT, bool SET>
 static int launch_map(size_t smem, int T, int lo, int hi, int target, int S, int ST, int C, const float* in,
                       float* out, cudaStream_t st) {
-    const auto kernel = accumulate_map_kernel<I, ADJOINT, SET>;
-    DS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 1;
-    DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMapWarps * 32, smem));
+    const int rc = resident_ctas<accumulate_map_kernel<I, ADJOINT, SET>>(kMapWarps * 32, smem, &per_sm);
+    if (rc) return rc;
     const int64_t want = ((int64_t)T + I * kMapWarps - 1) / (I * kMapWarps);
-    const int64_t wave = (int64_t)sm_count() * (per_sm < 1 ? 1 : per_sm);  // the tables are built once per CTA
-    kernel<<<(unsigned)(want < wave ? want : wave), kMapWarps * 32, smem, st>>>(T, lo, hi, target, S, ST, C, in, out);
+    const int64_t wave = (int64_t)sm_count() * per_sm;  // the tables are built once per CTA
+    accumulate_map_kernel<I, ADJOINT, SET><<<(unsigned)(want < wave ? want : wave), kMapWarps * 32, smem, st>>>(
+        T, lo, hi, target, S, ST, C, in, out);
     return check_launch("accumulate_to_level");
 }
 
