@@ -366,23 +366,6 @@ static bool lattice_tab_fits(int lo, int hi, int S, int ST, int CP) {
            (CP == 16 && lattice_tab_smem<16>(lo, hi, S, ST, false) <= 110 * 1024);
 }
 
-// The table kernels' dynamic shared memory above the 48 KB default, and
-// the CTAs of that size one SM holds (one record per kernel: the template
-// argument is the kernel itself).
-template <auto Kernel>
-static int tab_smem_attr(size_t smem, int* per_sm = nullptr) {
-    static size_t set = 0;
-    static int fit = 1;
-    if (smem != set) {
-        DS_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        DS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, Kernel, kMapWarps * 32, smem));
-        if (fit < 1) fit = 1;
-        set = smem;
-    }
-    if (per_sm) *per_sm = fit;
-    return DS_OK;
-}
-
 // clip[b][v] = mvp[b] . (verts[v], 1)  (examples/utils.py:412-426)
 __global__ void __launch_bounds__(kThreads) project_kernel(int B, int V, const float* __restrict__ verts,
                                                            const float* __restrict__ mvp, float* __restrict__ pos) {
@@ -877,7 +860,7 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
 #define DSB_TAB(KERNEL, BWD, EXTRA, CC, CPP, STREAM, ...)                                                          \
     do {                                                                                                           \
         const size_t tsm = lattice_tab_smem<CPP>(c.min_level, c.max_level, S, ST, BWD);                            \
-        int per_sm = 1, trc = tab_smem_attr<KERNEL<CC, CPP>>(tsm, &per_sm);                                        \
+        int per_sm = 1, trc = resident_ctas<KERNEL<CC, CPP>>(kMapWarps * 32, tsm, &per_sm);                        \
         if (trc) return trc;                                                                                       \
         const int per = kTabGroup<CPP> * (kMapWarps / kTabGroupWarps<CPP>); /* triangles of a CTA's pass */        \
         const int64_t want = ((int64_t)c.T + per - 1) / per;                                                       \

@@ -64,3 +64,22 @@ def i64(v: int):
 
 def stream():
     return C.c_void_p(STREAM)
+
+
+def feats(lo: int, hi: int) -> int:
+    return sum(3 if k == 0 else ((1 << k - 1) + 1) * ((1 << k) + 1) for k in range(lo, hi + 1))
+
+
+class StepConfig(C.Structure):
+    """ds_step_config of include/diffsoup_b200.h."""
+    _fields_ = [(n, C.c_float if n in ("thr_const", "frag_records") else C.c_int32) for n in
+                ("B", "T", "V", "C", "min_level", "max_level", "hidden", "n_layers", "stochastic", "thr_const",
+                 "frag_records", "precision", "block_shape", "view_enc", "target_u8", "shade_mode")]
+
+
+def train_step(B=2, T=3000, H=96, W=128, C_=8, hi=2, hidden=16, layers=1, frag_records=2.0, precision=1) -> list:
+    """The calls of one ds_train_step."""
+    c = StepConfig(B, T, 3 * T, C_, 0, hi, hidden, layers, 1, 0.5, frag_records, precision, 0, 0, 0, 0)
+    nt, cap = B * ((W + 15) // 16) * ((H + 15) // 16), i64(8 * B * T)
+    need = lib.ds_train_step_workspace_size(C.byref(c), nt, i64(B * H * W), cap)
+    return call("ds_train_step", C.byref(c), "p", nt, i64(B * H * W), *["p"] * 17, C.c_size_t(need), cap, "p", stream())

@@ -28,3 +28,18 @@ print("sizes", *smem)
     assert lines["inner"] == "0" and lines["outer"].split()[0] == "0", out
     small, large = map(int, lines["sizes"].split())
     assert small < large and large > 48 * 1024  # the two calls share a kernel and differ in size
+
+
+def test_training_step(tmp_path):
+    """Two steps of one model with other levels: a step's forward and adjoint kernels launch with their own sizes."""
+    out = run(tmp_path, """
+wide = dict(C_=16, hidden=64, layers=2, precision=0)
+train_step(hi=3, **wide)
+sizes = lambda log: sorted({int(x[3]) for x in log if x[0] == "launch" and "accum_tab" in x[4]})
+inner = C.CFUNCTYPE(None)(lambda: print("inner", *sizes(train_step(hi=2, **wide))))
+fake.fake_before_launch(inner)  # before the level accumulation, the step's first launch
+print("outer", *sizes(train_step(hi=3, **wide)))
+""")
+    lines = dict(line.split(" ", 1) for line in out.splitlines())
+    inner, outer = ([int(v) for v in lines[k].split()] for k in ("inner", "outer"))
+    assert inner and outer and inner[0] < outer[0] and inner[-1] < outer[-1]
