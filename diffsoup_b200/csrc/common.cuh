@@ -30,11 +30,13 @@ inline unsigned blocks_for(int64_t n, int threads = kThreads) {
 // captured step of 5,000 triangles 82 -> 81 us, resampling 1.13 -> 1.09 ms).  Every kernel launched this way
 // begins with chain_wait(), which returns when the kernel before it has
 // finished and its writes are visible; so it may read and overwrite what any earlier
-// kernel of the stream wrote or read.  Launches that follow an event wait use
-// <<<>>> (they have more than one kernel to wait for).
+// kernel of the stream wrote or read.  Only a kernel that follows a kernel, memset or
+// copy of the same call is chained.  After an event wait there is more than one
+// kernel to wait for, and what the caller put on the stream before the call is
+// not known: those launches are plain (chained = false, or <<<>>>).
 template <class... P, class... A>
-inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
-                           const A&... args) {
+inline void launch_kernel(bool chained, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                          const A&... args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -44,8 +46,14 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, si
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // errors: check_launch
+}
+
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                           const A&... args) {
+    launch_kernel(true, kernel, grid, threads, smem, st, args...);
 }
 
 // Waits for the kernel before this one (returns at once where none is pending), then lets the next one

@@ -23,6 +23,7 @@
 // interpolation and view encoding in FP32 as the shader, the MLP of a warp's 32
 // pixels on the tensor cores in 3xTF32 (FP32 accuracy, below).
 #include "geometry.cuh"
+#include "tiled.cuh"
 
 namespace dsb {
 
@@ -287,12 +288,12 @@ static int check_post_args(int B, const ds_view_desc* views, int64_t num_pixels,
 static int launch_post(int B, const ds_view_desc* views, int64_t num_pixels, const float* gbuf, int level,
                        const unsigned char* lut0, const unsigned char* lut1, int64_t num_texels,
                        const float* inv_mvp, const float* mlp_params, float bg_r, float bg_g, float bg_b, float* rgb,
-                       unsigned char* rgba8, cudaStream_t st) {
+                       unsigned char* rgba8, cudaStream_t st, bool chained) {
     if (num_pixels == 0) return DS_OK;
-    launch_chained(deferred_shade_kernel, dim3(pixel_grid(num_pixels)), kThreads, 0, st, B, views, num_pixels,
-                   reinterpret_cast<const float4*>(gbuf), level, (int)feats_at_level((uint32_t)level),
-                   reinterpret_cast<const uchar4*>(lut0), reinterpret_cast<const uchar4*>(lut1), num_texels, inv_mvp,
-                   mlp_params, bg_r, bg_g, bg_b, rgb, reinterpret_cast<uchar4*>(rgba8));
+    launch_kernel(chained, deferred_shade_kernel, dim3(pixel_grid(num_pixels)), kThreads, 0, st, B, views, num_pixels,
+                  reinterpret_cast<const float4*>(gbuf), level, (int)feats_at_level((uint32_t)level),
+                  reinterpret_cast<const uchar4*>(lut0), reinterpret_cast<const uchar4*>(lut1), num_texels, inv_mvp,
+                  mlp_params, bg_r, bg_g, bg_b, rgb, reinterpret_cast<uchar4*>(rgba8));
     return check_launch("render_deferred");
 }
 
@@ -322,7 +323,7 @@ int ds_render_deferred(int B, const ds_view_desc* views, int64_t num_pixels, con
                                    rgb, rgba8);
     if (rc) return rc;
     return launch_post(B, views, num_pixels, gbuf, level, lut0, lut1, num_texels, inv_mvp, mlp_params, bg_r, bg_g,
-                       bg_b, rgb, rgba8, (cudaStream_t)stream);
+                       bg_b, rgb, rgba8, (cudaStream_t)stream, false);
 }
 
 size_t ds_render_workspace_size(int B, int V, int T, int num_tiles, int64_t list_capacity) {
@@ -352,11 +353,11 @@ int ds_render_frame(int B, const ds_view_desc* views, int num_tiles, int64_t num
     if ((rc = ds_project_vertices(B, V, verts, mvp, pos, stream))) return rc;
     if ((rc = ds_tiles_bin(B, views, num_tiles, V, pos, T, faces, tiles, tiles_bytes, list_capacity, status, stream)))
         return rc;
-    if ((rc = ds_tiles_rasterize(B, views, num_tiles, V, pos, T, faces, level, S, alpha, 0, 0.5f, nullptr, gbuf,
-                                 tiles, tiles_bytes, list_capacity, stream)))
+    if ((rc = tiles_rasterize_impl(B, views, num_tiles, T, level, S, alpha, 0, 0.5f, nullptr, gbuf, tiles, list_capacity,
+                                   nullptr, st, kDefaultBlockShape, true)))
         return rc;
     return launch_post(B, views, num_pixels, gbuf, level, lut0, lut1, num_texels, inv_mvp, mlp_params, bg_r, bg_g,
-                       bg_b, rgb, rgba8, st);
+                       bg_b, rgb, rgba8, st, num_tiles > 0);
 }
 
 }  // extern "C"

@@ -951,7 +951,7 @@ int ds_train_step(const ds_step_config* cfg, const ds_view_desc* views, int num_
     // stream beside the edge gradients
     if (side && (rc = fork_to(side, 1, st))) return rc;
     rc = tiles_aux_impl(c.B, views, num_tiles, c.T, c.max_level, ST, w.alpha_acc, w.l1, rast, a.inv_n,
-                        w.grad_alpha_acc, w.tiles, list_capacity, rs, sst, block_shape_log2(c));
+                        w.grad_alpha_acc, w.tiles, list_capacity, rs, sst, block_shape_log2(c), side == nullptr);
     if (rc) return rc;
     if (side && (rc = accum_backward(sst))) return rc;
     if ((rc = mark(5, st))) return rc;

@@ -1059,25 +1059,15 @@ int tiles_rasterize_impl(int B, const ds_view_desc* views, int num_tiles, int T,
     if (rs != nullptr) {
         const void* k = reinterpret_cast<const void*>(&raster_kernel<true>);
         const dim3 grid(block_grid(num_tiles, k, g_occ_raster_rec));
-        if (chained)
-            launch_chained(raster_kernel<true>, grid, kWarpsPerCta * 32, 0, st, B, views, num_tiles, T, w.boxes, w.verts,
-                           w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, thr_mode, thr_const,
-                           rng, w.work, rast, *rs, bwl);
-        else
-            raster_kernel<true><<<grid, kWarpsPerCta * 32, 0, st>>>(
-                B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
-                alpha_src, thr_mode, thr_const, rng, w.work, rast, *rs, bwl);
+        launch_kernel(chained, raster_kernel<true>, grid, kWarpsPerCta * 32, 0, st, B, views, num_tiles, T, w.boxes,
+                      w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, thr_mode,
+                      thr_const, rng, w.work, rast, *rs, bwl);
     } else {
         const void* k = reinterpret_cast<const void*>(&raster_kernel<false>);
         const dim3 grid(block_grid(num_tiles, k, g_occ_raster));
-        if (chained)
-            launch_chained(raster_kernel<false>, grid, kWarpsPerCta * 32, 0, st, B, views, num_tiles, T, w.boxes, w.verts,
-                           w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, thr_mode, thr_const,
-                           rng, w.work, rast, RecordStore{}, bwl);
-        else
-            raster_kernel<false><<<grid, kWarpsPerCta * 32, 0, st>>>(
-                B, views, num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S,
-                alpha_src, thr_mode, thr_const, rng, w.work, rast, RecordStore{}, bwl);
+        launch_kernel(chained, raster_kernel<false>, grid, kWarpsPerCta * 32, 0, st, B, views, num_tiles, T, w.boxes,
+                      w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, thr_mode,
+                      thr_const, rng, w.work, rast, RecordStore{}, bwl);
     }
     return check_launch("tiles_rasterize");
 }
@@ -1085,12 +1075,12 @@ int tiles_rasterize_impl(int B, const ds_view_desc* views, int num_tiles, int T,
 static int aux_launch(int B, const ds_view_desc* views, int num_tiles, int T, int level, int S,
                       const float* alpha_src, int C, const float* color, const float* target, const float* rast,
                       float scale, float* grad_alpha_src, void* workspace, int64_t list_capacity,
-                      const int* item_list, const int* item_count, cudaStream_t st, int bwl) {
+                      const int* item_list, const int* item_count, cudaStream_t st, int bwl, bool chained) {
     TileWs w = carve(workspace, B, T, num_tiles, list_capacity, nullptr);
     const void* k = reinterpret_cast<const void*>(&aux_kernel);
-    launch_chained(aux_kernel, dim3(block_grid(num_tiles, k, g_occ_aux)), kWarpsPerCta * 32, 0, st, B, views, num_tiles, T,
-                   w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src, C, color,
-                   target, rast, scale, item_list, item_count, w.work + 1, grad_alpha_src, bwl);
+    launch_kernel(chained, aux_kernel, dim3(block_grid(num_tiles, k, g_occ_aux)), kWarpsPerCta * 32, 0, st, B, views,
+                  num_tiles, T, w.boxes, w.verts, w.edges, w.offsets, w.sorted, w.list, list_capacity, level, S, alpha_src,
+                  C, color, target, rast, scale, item_list, item_count, w.work + 1, grad_alpha_src, bwl);
     return check_launch("tiles_opacity_aux");
 }
 
@@ -1101,16 +1091,16 @@ TileTables tiles_tables(void* workspace, int B, int T, int num_tiles, int64_t li
 
 int tiles_aux_impl(int B, const ds_view_desc* views, int num_tiles, int T, int level, int S, const float* alpha_src,
                    const float* l1, const float* rast, float scale, float* grad_alpha_src, void* workspace,
-                   int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl) {
+                   int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl, bool chained) {
     if (num_tiles == 0) return DS_OK;
     if (rs == nullptr)
         return aux_launch(B, views, num_tiles, T, level, S, alpha_src, 1, l1, nullptr, rast, scale, grad_alpha_src,
-                          workspace, list_capacity, nullptr, nullptr, st, bwl);
+                          workspace, list_capacity, nullptr, nullptr, st, bwl, chained);
     aux_records_kernel<<<sm_count() * 8, kRecChunk, 0, st>>>(*rs, level, S, alpha_src, l1, scale, grad_alpha_src);
     const int rc = check_launch("tiles_opacity_aux records");
     if (rc) return rc;
     return aux_launch(B, views, num_tiles, T, level, S, alpha_src, 1, l1, nullptr, rast, scale, grad_alpha_src,
-                      workspace, list_capacity, rs->fallback, rs->counters + 1, st, bwl);
+                      workspace, list_capacity, rs->fallback, rs->counters + 1, st, bwl, true);
 }
 
 }  // namespace dsb
@@ -1128,7 +1118,7 @@ int ds_tiles_rasterize(int B, const ds_view_desc* views, int num_tiles, int V, c
     DS_CHECK_ARG(thr_mode == 0 || (thr_mode == 1 && rng != nullptr), "tiles_rasterize: bad threshold mode");
     DS_CHECK_ARG(((uintptr_t)rast & 15) == 0, "tiles_rasterize: rast not 16-byte aligned");
     return tiles_rasterize_impl(B, views, num_tiles, T, level, S, alpha_src, thr_mode, thr_const, rng, rast,
-                                workspace, list_capacity, nullptr, (cudaStream_t)stream, kDefaultBlockShape, true);
+                                workspace, list_capacity, nullptr, (cudaStream_t)stream, kDefaultBlockShape, false);
 }
 
 int ds_tiles_opacity_aux(int B, const ds_view_desc* views, int num_tiles, int V, const float* pos, int T,
@@ -1144,7 +1134,7 @@ int ds_tiles_opacity_aux(int B, const ds_view_desc* views, int num_tiles, int V,
     DS_CHECK_ARG(((uintptr_t)rast & 15) == 0, "tiles_opacity_aux: rast not 16-byte aligned");
     if (num_tiles == 0) return DS_OK;
     return aux_launch(B, views, num_tiles, T, level, S, alpha_src, C, color, target, rast, scale, grad_alpha_src,
-                      workspace, list_capacity, nullptr, nullptr, (cudaStream_t)stream, kDefaultBlockShape);
+                      workspace, list_capacity, nullptr, nullptr, (cudaStream_t)stream, kDefaultBlockShape, false);
 }
 
 }  // extern "C"

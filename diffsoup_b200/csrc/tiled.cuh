@@ -66,17 +66,16 @@ struct RecordStore {
 constexpr int kDefaultBlockShape = 3;
 
 // Rasterizer of ds_tiles_rasterize; records fragments when rs != nullptr.
-// chained: launched with launch_chained (not right after an event wait).
+// chained: see launch_kernel.
 int tiles_rasterize_impl(int B, const ds_view_desc* views, int num_tiles, int T, int level, int S,
                          const float* alpha_src, int thr_mode, float thr_const, const uint64_t* rng, float* rast,
                          void* workspace, int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl, bool chained);
 
 // Opacity auxiliary gradient with a per-pixel loss l1 [pixels]: from the
 // records plus the fallback blocks when rs != nullptr, else by
-// re-enumerating every block.
+// re-enumerating every block.  chained (without records): see launch_kernel.
 int tiles_aux_impl(int B, const ds_view_desc* views, int num_tiles, int T, int level, int S, const float* alpha_src,
                    const float* l1, const float* rast, float scale, float* grad_alpha_src, void* workspace,
-                   int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl);
-
+                   int64_t list_capacity, const RecordStore* rs, cudaStream_t st, int bwl, bool chained);
 
 }  // namespace dsb
