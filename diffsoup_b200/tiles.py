@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes as C
 import itertools
+import threading
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -61,13 +62,16 @@ def view_table(hw: Sequence[Tuple[int, int]], device: torch.device):
 # taken again only shows an older call's status.
 _SLOTS = 256
 _slots: List = []  # [tensor, ctypes view], once allocated
+_slots_lock = threading.Lock()
 _next_slot = itertools.count()
 
 
 def _status_slots():
     if not _slots:
-        t = torch.full((_SLOTS,), -1, dtype=torch.int32, pin_memory=True)
-        _slots[:] = [t, (C.c_int32 * _SLOTS).from_address(t.data_ptr())]
+        with _slots_lock:  # once: the device may still write to a ring that a second one would replace
+            if not _slots:
+                t = torch.full((_SLOTS,), -1, dtype=torch.int32, pin_memory=True)
+                _slots[:] = [t, (C.c_int32 * _SLOTS).from_address(t.data_ptr())]
     return _slots
 
 
