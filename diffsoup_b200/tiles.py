@@ -75,14 +75,6 @@ def _status_slots():
     return _slots
 
 
-def copy_status(status: torch.Tensor):
-    """Queues a copy of a status word (int32 [1], device) to the host; the returned
-    function reads it once the stream has been synchronised."""
-    slots, slot = _status_slots(), next(_next_slot) % _SLOTS
-    slots[0][slot:slot + 1].copy_(status, non_blocking=True)
-    return lambda: int(slots[1][slot])
-
-
 def _device_index(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 

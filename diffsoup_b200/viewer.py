@@ -173,9 +173,9 @@ class Renderer:
             out.append(f.rgb.view(f.B, f.H, f.W, 3).clone())
         if gbuf:
             out.append(f.gbuf.view(f.B, f.H, f.W, 4).clone())
-        status = _tiles.copy_status(f.status)
+        f.status_host.copy_(f.status, non_blocking=True)
         torch.cuda.current_stream(self.device).synchronize()
-        if status() & _tiles.DS_STATUS_LIST_OVERFLOW:
+        if int(f.status_host) & _tiles.DS_STATUS_LIST_OVERFLOW:
             f.grow()  # this frame is exact all the same; the next ones bin without overflow
         return out[0] if len(out) == 1 else tuple(out)
 
@@ -211,6 +211,7 @@ class _Frame:
             self.rgb = torch.empty(self.num_pixels, 3, dtype=torch.float32, device=dev)
             self.rgba8 = torch.empty(self.num_pixels, 4, dtype=torch.uint8, device=dev)
             self.status = torch.zeros(1, dtype=torch.int32, device=dev)
+            self.status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)  # render()'s copy of it
         self.capacity = max(1 << 16, 8 * B * r.T)
         self._alloc()
 
