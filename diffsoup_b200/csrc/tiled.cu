@@ -1024,7 +1024,8 @@ int ds_tiles_bin_report(int B, const ds_view_desc* views, int num_tiles, int V, 
     const int rc = ds_tiles_bin(B, views, num_tiles, V, pos, T, tri, workspace, workspace_bytes, list_capacity, status,
                                 stream);
     if (rc) return rc;
-    DS_CUDA(cudaMemcpyAsync(status_host, status, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    if (status_host != nullptr)
+        DS_CUDA(cudaMemcpyAsync(status_host, status, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     return DS_OK;
 }
 

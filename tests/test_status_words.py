@@ -6,6 +6,7 @@ import time
 import pytest
 import torch
 
+import diffsoup_b200 as ds
 from diffsoup_b200 import scenes, tiles, viewer
 
 
@@ -55,3 +56,24 @@ def test_a_frame_reads_its_own_status(monkeypatch):
     frame.capacity = 8
     frame._alloc()
     assert torch.equal(r.render(vi.mvps, 64, 80), want) and frame.capacity == 16
+
+
+@pytest.mark.gpu
+def test_replays_leave_the_ring_alone():
+    """A captured call's replays write into no word of the ring, which later calls have by then."""
+    sc = scenes.make_scene(2, seed=2, num_tris=300, num_views=1, resolution=(48, 64), with_targets=False)
+    pos = torch.from_numpy(sc.clip_positions()).cuda()
+    tri, alpha = torch.from_numpy(sc.tri).cuda(), torch.rand(sc.T, 15, 1, device="cuda")
+    call = lambda: ds.rasterize_multires_triangle_alpha((48, 64), pos, tri, 2, alpha, stochastic=False)  # noqa: E731
+    want = call()
+    graph = torch.cuda.CUDAGraph()
+    tiles._last = None
+    with torch.cuda.graph(graph):
+        got = call()
+    words = tiles._status_slots()[1]
+    words[:] = [77] * len(words)
+    got.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and set(words) == {77}
+    call()
