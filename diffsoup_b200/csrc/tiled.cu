@@ -638,12 +638,14 @@ __device__ __forceinline__ unsigned warp_transpose(unsigned m) {
 // meets the block, whose depth bound passes `zcut` and that may cover one of its
 // valid pixels, and returns the calling lane's pixel's candidates as a mask over
 // the group.  *head_zlo receives the zlo of the group's first entry (the
-// smallest, when the list is ordered).
+// smallest, when the list is ordered); *any_large whether a staged triangle's rect
+// has `large` pixels or more.
 __device__ __forceinline__ unsigned stage_pixels(const BlockGeom& g, int64_t g0, const TriBox* __restrict__ boxes,
                                                  const TriVerts* __restrict__ verts,
                                                  const TriEdges* __restrict__ edges,
                                                  const ListEntry* __restrict__ list, int T, float zcut, unsigned valid,
-                                                 RasterStage& st, float* head_zlo) {
+                                                 RasterStage& st, float* head_zlo, int large = 0x7fffffff,
+                                                 bool* any_large = nullptr) {
     const int lane = threadIdx.x & 31;
     const int64_t e = g0 + lane;
     const bool in = e < g.end;
@@ -672,6 +674,8 @@ __device__ __forceinline__ unsigned stage_pixels(const BlockGeom& g, int64_t g0,
         st.t[lane] = ri - g.b * T;
     }
     __syncwarp();
+    if (any_large != nullptr)
+        *any_large = __any_sync(0xffffffffu, lanes != 0u && (bx.y1 - bx.y0) * (bx.x1 - bx.x0) >= large);
     return warp_transpose(lanes);
 }
 
@@ -806,12 +810,27 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, DSB_RASTER_MIN_CTAS) raster
     if (REC && cid >= 0 && lane == 0) rs.chunk_fill[cid] = cfill;
 }
 
-// dL/dalpha of one fragment scattered through the lattice adjoint
-// (rasterize.cu:951-970 followed by multires.cu:130-222).
-__device__ __forceinline__ void aux_scatter(float b0, float b1, int level, int S, const float* __restrict__ alpha_src,
-                                            int t, float loss, bool visible, float scale,
-                                            float* __restrict__ grad_alpha_src) {
-    uint32_t idx[3];
+// Opacity contributions in the re-enumerating pass.  About one fragment a pixel is
+// in front of its surface, far below the atomics' rate, so most go straight to
+// memory.  The atomics of a large triangle, though, meet on its few samples: 20 ms for
+// two triangles over 8 views of 800x800 at level 2.  So where one of the 32 list entries that
+// a warp stages is a triangle of kAuxLarge pixels of its rect or more per sample, the warp's fragments are
+// summed before the atomics: those on one triangle (kAuxSameTriangle lanes or more) in one lattice
+// cell (kAuxSameCell or more).  The two triangles then take 0.30 ms (0.34 with a warp's sums
+// in shared memory, for every triangle), 20 nearly transparent layers over one view 10 -> 0.20 ms (0.59), 200
+// triangles of 240 pixels' size in two views 20 -> 0.68 ms at level 0 (1.71).  Summed everywhere, two views of
+// 803x601 of 15,000 triangles take 71 us and 61 without any sums: 66 so (124).  Between them, 2,000 triangles of 80
+// pixels' size at level 4 take 59 us summed, 85 by this line and 109 by one twice as far (88); 12 and 6 lanes
+// instead of 8 and 4 take 1,056 us for the 200 triangles' 690.
+constexpr int kAuxLarge = 170;
+constexpr int kAuxSameTriangle = 8;
+constexpr int kAuxSameCell = 4;
+
+// dL/dalpha of one fragment through the lattice adjoint (rasterize.cu:951-970
+// followed by multires.cu:130-222): three samples idx and their contributions g.
+__device__ __forceinline__ void aux_contributions(float b0, float b1, int level, int S,
+                                                  const float* __restrict__ alpha_src, int t, float loss, bool visible,
+                                                  float scale, uint32_t idx[3], float g[3]) {
     float w[3];
     lattice_cell(b0, b1, level, idx, w);
     const float* src = alpha_src + (size_t)t * S;  // interp_level (the same sum)
@@ -819,9 +838,61 @@ __device__ __forceinline__ void aux_scatter(float b0, float b1, int level, int S
 #pragma unroll
     for (int q = 0; q < 3; ++q) alpha = madd(alpha, w[q], __ldg(src + idx[q]));
     const float ga = aux_alpha_grad(loss, alpha, visible) * scale;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) g[q] = ga * w[q];
+}
+
+__device__ __forceinline__ void aux_scatter(float b0, float b1, int level, int S, const float* __restrict__ alpha_src,
+                                            int t, float loss, bool visible, float scale,
+                                            float* __restrict__ grad_alpha_src) {
+    uint32_t idx[3];
+    float g[3];
+    aux_contributions(b0, b1, level, S, alpha_src, t, loss, visible, scale, idx, g);
     float* dst = grad_alpha_src + (size_t)t * S;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) atomicAdd(dst + idx[q], ga * w[q]);
+    for (int q = 0; q < 3; ++q) atomicAdd(dst + idx[q], g[q]);
+}
+
+// The same for the warp's fragments (one a lane, where `hit`; called by the whole
+// warp), those of one triangle and lattice cell summed before the atomics.
+__device__ __forceinline__ void aux_scatter_merged(bool hit, float b0, float b1, int level, int S,
+                                                   const float* __restrict__ alpha_src, int t, float loss,
+                                                   bool visible, float scale, float* __restrict__ grad_alpha_src) {
+    const int lane = threadIdx.x & 31;
+    uint32_t idx[3] = {0u, 0u, 0u};
+    float g[3] = {0.f, 0.f, 0.f};
+    if (hit) aux_contributions(b0, b1, level, S, alpha_src, t, loss, visible, scale, idx, g);
+    const unsigned mates = __match_any_sync(0xffffffffu, hit ? t : -1);  // the lanes on this lane's triangle
+    if (__any_sync(0xffffffffu, hit && __popc(mates) >= kAuxSameTriangle)) {
+        // a cell is its first sample and where the third lies to the first two
+        const uint32_t cell = idx[0] << 2 | (idx[2] == idx[0] ? 2u : (idx[2] > idx[1] ? 1u : 0u));
+        const unsigned peers = __match_any_sync(0xffffffffu, cell) & mates;
+        const bool merged = hit && __popc(peers) >= kAuxSameCell;
+        for (unsigned leaders = __ballot_sync(0xffffffffu, merged && lane == __ffs(peers) - 1); leaders != 0u;
+             leaders &= leaders - 1u) {
+            const int leader = __ffs(leaders) - 1;
+            const bool mine = (__shfl_sync(0xffffffffu, peers, leader) >> lane) & 1u;
+            const float v0 = mine ? g[0] : 0.f, v1 = mine ? g[1] : 0.f, v2 = mine ? g[2] : 0.f;
+            // sums over the warp, sum q in the lanes of quarter q
+            const bool hi = lane & 16, odd = lane & 8;
+            const float a = (hi ? v2 : v0) + __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, 16);
+            const float b = (hi ? 0.f : v1) + __shfl_xor_sync(0xffffffffu, hi ? v1 : 0.f, 16);
+            float v = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const uint32_t i0 = __shfl_sync(0xffffffffu, idx[0], leader), i1 = __shfl_sync(0xffffffffu, idx[1], leader),
+                           i2 = __shfl_sync(0xffffffffu, idx[2], leader);
+            const int lt = __shfl_sync(0xffffffffu, t, leader);
+            // three lanes in one instruction: samples of one 32-byte sector are one access
+            if ((lane & 7) == 0 && lane < 24)
+                atomicAdd(grad_alpha_src + (size_t)lt * S + (hi ? i2 : (odd ? i1 : i0)), v);
+        }
+        hit = hit && !merged;
+    }
+    if (!hit) return;
+    float* dst = grad_alpha_src + (size_t)t * S;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) atomicAdd(dst + idx[q], g[q]);
 }
 
 // Opacity auxiliary gradient from the fragment records: one thread per
@@ -885,11 +956,7 @@ __global__ void __launch_bounds__(kRecChunk) aux_records_kernel(RecordStore rs, 
 // recomputed and dL/dalpha is scattered through the lattice adjoint.
 // Fragments behind the visible surface contribute nothing
 // (rasterize.cu:950), so triangles whose depth bound lies behind every
-// lane's surface are never staged.  A fragment's three contributions go
-// straight to memory: about one fragment a pixel is in front of its surface, far below
-// the atomics' rate (summing a warp's contributions in shared memory first, with its
-// compare-and-swap loops, took 124 us against 79 us for two views of 803x601; per-pixel
-// candidates as in the rasterizer then gave 65 us).
+// lane's surface are never staged.
 // With item_list, only the blocks listed there (*item_count of them) are processed.
 __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
     int B, const ds_view_desc* __restrict__ views, int num_tiles, int T, const TriBox* __restrict__ boxes,
@@ -927,21 +994,28 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) aux_kernel(
         // the surface's depth (+inf where a valid pixel is empty) and the block's farthest
         const float z_cut = !g.valid ? -INFINITY : (tp >= 0 ? zp : INFINITY);
         const float warp_far = warp_max(z_cut);
+        const int large = kAuxLarge * S;
         for (int64_t g0 = g.begin; g0 < g.end; g0 += 32) {
             float head;
-            unsigned todo = stage_pixels(g, g0, boxes, verts, edges, list, T, warp_far, valid, st, &head);
+            bool merge;
+            unsigned todo = stage_pixels(g, g0, boxes, verts, edges, list, T, warp_far, valid, st, &head, large, &merge);
             if (g.ordered && head > warp_far) break;
             while (__any_sync(0xffffffffu, todo != 0u)) {
                 const int k = todo != 0u ? __ffs(todo) - 1 : 0;
                 // the pixel's surface does not lie in front of the triangle
                 const bool near = todo != 0u && !(st.zlo[k] > z_cut);
                 todo = !near && g.ordered ? 0u : todo & (todo - 1u);
-                if (!near) continue;
+                if (!merge && !near) continue;
                 const int t = st.t[k];
                 const float4 p0 = st.v[k].p0, p1 = st.v[k].p1, p2 = st.v[k].p2;
-                float b0, b1, depth;
-                if (fragment_at(ndc_y, ndc_x, p0, p1, p2, b0, b1, depth) && !(tp >= 0 && depth > zp))
-                    aux_scatter(b0, b1, level, S, alpha_src, t, loss, tp >= 0 && t == tp, scale, grad_alpha_src);
+                float b0 = 0.f, b1 = 0.f, depth;
+                const bool hit = near && fragment_at(ndc_y, ndc_x, p0, p1, p2, b0, b1, depth) && !(tp >= 0 && depth > zp);
+                const bool visible = tp >= 0 && t == tp;
+                if (!merge) {
+                    if (hit) aux_scatter(b0, b1, level, S, alpha_src, t, loss, visible, scale, grad_alpha_src);
+                } else if (__any_sync(0xffffffffu, hit)) {
+                    aux_scatter_merged(hit, b0, b1, level, S, alpha_src, t, loss, visible, scale, grad_alpha_src);
+                }
             }
             __syncwarp();
         }
