@@ -291,6 +291,11 @@ __global__ void __launch_bounds__(kThreads) color_backward_kernel(int64_t n, con
 // per pixel.  4 views of 800x800, 7 channels: 103 -> 43 us.
 constexpr int kMergeRow = 32;  // channels up to which the rows are staged
 
+// Floats between the staged rows: the row and its three weights, an odd number of floats, or of
+// groups of four, so that the rows of eight lanes fall in different banks (12 channels 88 us with 16 floats,
+// 72 with 20).
+__host__ __device__ constexpr int merge_stride(int C) { return C == 7 ? 11 : C + 4 + (C & 4); }
+
 template <bool ROW7>
 __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, int W, int bx, int64_t blocks, int per_view,
                                                                         const float* __restrict__ rast,
@@ -301,7 +306,7 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t block = (int64_t)blockIdx.x * (kThreads / 32) + warp;
     if (block >= blocks) return;  // warp-uniform
-    const int stride = ROW7 ? 11 : C + 4;  // the row and its three weights
+    const int stride = merge_stride(C);
     float* rows = merge_smem + (size_t)warp * (32 * stride + 160);
     int* meta = reinterpret_cast<int*>(rows + 32 * stride);
     const int64_t b = block / per_view;
@@ -335,9 +340,19 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
         covered ? ((unsigned long long)(unsigned)t << 34) | ((unsigned long long)(idx[0] & 0xffffu) << 18) |
                       ((unsigned long long)(idx[1] & 0xffffu) << 2) | (idx[2] == idx[0] ? 2u : (idx[2] > idx[1] ? 1u : 0u))
                 : ~0ull;
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    const bool leader = covered && lane == __ffs(peers) - 1;
-    const unsigned leaders = __ballot_sync(0xffffffffu, leader);
+    // where few pixels share a cell with the pixel beside or above them, the grouping is not tried: it is slow
+    // for many different keys (60,000 triangles, one a pixel, two views of 800x800, 4 channels: 34 us without
+    // grouping, 41 with it, 29 so; 8 channels 47, 54, 47)
+    const unsigned long long beside = __shfl_down_sync(0xffffffffu, key, 1), above = __shfl_down_sync(0xffffffffu, key, 8);
+    const int pairs = __popc(__ballot_sync(0xffffffffu, covered && (lane & 7) != 7 && beside == key)) +
+                      __popc(__ballot_sync(0xffffffffu, covered && lane < 24 && above == key));
+    unsigned peers = 0u, leaders = live;
+    bool leader = false;
+    if (6 * pairs >= __popc(live)) {
+        peers = __match_any_sync(0xffffffffu, key);
+        leader = covered && lane == __ffs(peers) - 1;
+        leaders = __ballot_sync(0xffffffffu, leader);
+    }
     const int groups = __popc(leaders);
     if (3 * groups > 2 * __popc(live)) {
         if (!covered) return;
@@ -616,8 +631,7 @@ int ds_backward_multires_triangle_color(int B, int H, int W, const float* rast, 
     const int64_t nb = (int64_t)B * bx * by;
     if (min_level == max_level && max_level <= 8 && C <= kMergeRow && (vec || (C == 7 && aligned16(grad_features))) &&
         (int64_t)bx * by <= 0x7fffffff && nb <= 0x7fffffff) {
-        const int stride = C == 7 ? 11 : C + 4;
-        const size_t smem = (size_t)(kThreads / 32) * (32 * stride + 160) * sizeof(float);
+        const size_t smem = (size_t)(kThreads / 32) * (32 * merge_stride(C) + 160) * sizeof(float);
         const unsigned grid = (unsigned)((nb + kThreads / 32 - 1) / (kThreads / 32));
         if (C == 7)
             color_backward_merge_kernel<true><<<grid, kThreads, smem, st>>>(H, W, bx, nb, bx * by, rast, max_level, S, C,
