@@ -256,8 +256,9 @@ __device__ __forceinline__ void map_triangles(const MapTables& m, int t0, int T,
 }
 
 // Triangles per warp pass: as many of 4, 2, 1 as keep the warp's tile of
-// n_in elements at most 12 KB (8 warps and the tables then leave room for two
-// CTAs per SM); 0 when one triangle does not fit in 24 KB.
+// n_in elements at most 12 KB (with 8 warps' tiles of that size and the tables of levels 0..2
+// two CTAs share an SM, with those of levels 0..4 one has it alone); 0 when
+// one triangle does not fit in 24 KB.
 __host__ inline int map_interleave(int n_in) {
     if (n_in * 16 <= 12 * 1024) return 4;
     if (n_in * 8 <= 12 * 1024) return 2;

@@ -464,11 +464,23 @@ __global__ void __launch_bounds__(kThreads) accumulate_forward_kernel(int T, uin
     }
 }
 
+// Zeroes n floats, a group of four a thread (1.8 MB and the additions of 153,000 samples after it: 10.3 us, with
+// a memset 12.2).
+__global__ void __launch_bounds__(kThreads) zero_floats_kernel(int64_t n, float* __restrict__ p) {
+    const int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
+    if (i + 4 <= n && ((uintptr_t)p & 15) == 0) {
+        *reinterpret_cast<float4*>(p + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+        for (int64_t k = i; k < i + 4 && k < n; ++k) p[k] = 0.f;
+    }
+}
+
 // multires.cu:393-430
 __global__ void __launch_bounds__(kThreads) accumulate_backward_kernel(int T, uint32_t lo, uint32_t hi,
                                                                        uint32_t target, uint32_t S, uint32_t ST, int C,
                                                                        float* __restrict__ grad_feat,
                                                                        const float* __restrict__ grad_out) {
+    chain_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)T * ST) return;
     const uint32_t t = (uint32_t)(i / ST), k = (uint32_t)(i % ST);
@@ -494,19 +506,31 @@ __global__ void __launch_bounds__(kThreads) accumulate_backward_kernel(int T, ui
 static bool levels_ok(int lo, int hi) { return lo >= 0 && hi >= lo && hi <= 12; }
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// The map's tables and tiles in shared memory, or 0 where the kernels of one
-// thread per target sample run: lattices whose pairs or samples outgrow shared
-// memory (beyond levels 0..4 with 16 channels or so), and calls of fewer than
-// kMapMinSamples target samples, which end before the tables are built.
-constexpr int64_t kMapMinSamples = 2048;
+// The map's tables and tiles in shared memory, or *interleave = 0 where the
+// kernels of one thread per target sample run: lattices whose pairs or samples
+// outgrow shared memory (beyond levels 0..4 with 16 channels or so), and calls in which those kernels are
+// faster.  The lines were laid between 1,791 forms timed on both sides (22 ranges of levels, 1 to 128 channels, 10 to
+// 100,000 triangles); on their side of them, those that take the map lose to the other kernel by at most 2.5 us:
+//   * both: the map reads all S samples of a triangle and the other kernel only the N pairs' (levels 0..5 at level 2,
+//     30,000 triangles of 7 channels: N = 270, S = 783, forward 270 us against 102);
+//   * forward: less than a pass of one CTA an SM leaves SMs idle while the others build the tables (levels 2..2 at level 4,
+//     100 triangles of 8 channels: 18.6 against 6.3 us), and a few values a triangle are not worth the tables at all
+//     (level 0, 100,000 triangles of 3 channels: 10.4 against 6.7 us);
+//   * adjoint: kMapMinProducts atomic additions (of three) end before the tables are built (level 4, 3,000 triangles of 3
+//     channels: 19.1 against 16.6 us; of 4 channels 20.6 against 22.7).
 constexpr int kMapMaxPairs = 2400;
+constexpr int kMapMinValues = 32;
+constexpr int64_t kMapMinProducts = 1500000;
 
 static size_t map_smem_bytes(int64_t T, int lo, int hi, int S, int ST, int C, bool adjoint, int* interleave) {
     *interleave = 0;
-    if (T * ST < kMapMinSamples || (int64_t)ST * (hi - lo + 1) * 3 > kMapMaxPairs) return 0;
-    if ((int64_t)(S > ST ? S : ST) * C > 6 * 1024) return 0;
-    const int N = ST * (hi - lo + 1) * 3, n_in = (adjoint ? ST : S) * C;
-    *interleave = map_interleave(n_in);
+    const int NL = hi - lo + 1;
+    if ((int64_t)ST * NL * 3 > kMapMaxPairs || (int64_t)(S > ST ? S : ST) * C > 6 * 1024) return 0;
+    const int N = ST * NL * 3, n_in = (adjoint ? ST : S) * C, I = map_interleave(n_in);
+    if (adjoint ? 2 * N < S || T * ST * NL * C < kMapMinProducts
+                : 4 * N < 5 * S || T < (int64_t)I * kMapWarps * sm_count() || ST * NL * C < kMapMinValues)
+        return 0;
+    *interleave = I;
     return map_table_bytes(N, adjoint ? S : ST) + (size_t)kMapWarps * n_in * *interleave * sizeof(float);
 }
 
@@ -546,9 +570,10 @@ static int accumulate_backward(bool set, int T, int min_level, int max_level, in
                                                 grad_out, grad_features, st)
                    : launch_map_any<true, false>(interleave, smem, T, min_level, max_level, target_level, S, S_target,
                                                  C, grad_out, grad_features, st);
-    if (set) DS_CUDA(cudaMemsetAsync(grad_features, 0, (size_t)T * S * C * sizeof(float), st));
-    accumulate_backward_kernel<<<blocks_for(n), kThreads, 0, st>>>(T, min_level, max_level, target_level, S, S_target,
-                                                                   C, grad_features, grad_out);
+    const int64_t floats = (int64_t)T * S * C;
+    if (set) zero_floats_kernel<<<blocks_for((floats + 3) / 4), kThreads, 0, st>>>(floats, grad_features);
+    launch_kernel(set, accumulate_backward_kernel, dim3(blocks_for(n)), kThreads, 0, st, T, min_level, max_level,
+                  target_level, S, S_target, C, grad_features, grad_out);
     return check_launch("accumulate_to_level_backward");
 }
 

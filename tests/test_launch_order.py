@@ -28,6 +28,7 @@ CALLS = {
                     " NT, i64(9600))), i64(9600), 'p', stream())",
     "split_count": "call('ds_split_soup_count', 0, None, 1.0, 0.1, -1, 900, 'p', 300, 'p', None, 'p', C.byref(i64(0)),"
                    " 'p', C.c_size_t(lib.ds_split_soup_workspace_size(300)), 'p', stream())",
+    "levels_backward": "call('ds_accumulate_to_level_backward_set', 100, 0, 2, 2, 24, 15, 7, 'p', 'p', stream())",
     "triangle_rects": "call('ds_compute_triangle_rects', 96, 48, 2, 900, 'p', 300, 'p', 'p', 'p', C.byref(C.c_int(0)),"
                       " 'p', C.c_size_t(1 << 20), stream())",
 }

@@ -16,11 +16,11 @@ def p(v): import ctypes; return ctypes.c_void_p(v)
 
 def test_level_operators(tmp_path):
     out = run(tmp_path, LEVELS + """
-assert forward(2000, 3, 7) == 0
+assert forward(20000, 3, 7) == 0
 fake.fake_take()
-inner = C.CFUNCTYPE(None)(lambda: print("inner", forward(5000, 2, 1)))
+inner = C.CFUNCTYPE(None)(lambda: print("inner", forward(50000, 2, 1)))
 fake.fake_before_launch(inner)
-print("outer", forward(2000, 3, 7), lib.ds_last_error().decode())
+print("outer", forward(20000, 3, 7), lib.ds_last_error().decode())
 smem = [int(l.split()[3]) for l in fake.fake_take().decode().splitlines() if l.startswith("launch")]
 print("sizes", *smem)
 """)
