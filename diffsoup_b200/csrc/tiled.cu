@@ -133,10 +133,11 @@ __device__ __forceinline__ void warp_items(int n, F&& f) {
 // Triangles per warp of the two binning passes.  A warp's time is a chain of
 // items / 32 dependent rounds, so when 32 triangles a warp would leave most of
 // the chip without a warp, a warp takes 8 (its first lanes own one each, all
-// lanes work on their tiles).  At 15,000 pairs (one 1200x1200 view) 8 a warp
-// took the two passes from 59 to 22 us (with the fill pass below); at 120,000
-// (8 views of 800x800) 32 a warp took 43 us and 8 a warp 57 us.
-constexpr int64_t kBinNarrow = 60000;  // (view, triangle) pairs up to which a warp takes 8
+// lanes work on their tiles).  Whole binning with 8 and with 32 a warp, in us: one view of 800x800 of
+// 15,000 triangles 35 and 38, of 24,000 40 and 43, of 27,000 47.5 and 47.5, of 45,000 62 and 60, of 60,000 76 and 62;
+// one of 1200x1200 of 15,000 40 and 52; 4 views of 300x300 of 20,000 74 and 51; 200,000 triangles in
+// full HD 78 and 52.
+constexpr int64_t kBinNarrow = 24000;  // (view, triangle) pairs up to which a warp takes 8
 
 // Record index of the calling lane, or n for a lane without one.
 template <int TPW>
