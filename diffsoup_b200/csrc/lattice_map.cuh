@@ -202,9 +202,9 @@ struct MapVec<4> { typedef float4 type; };
 // element e of triangle t is src(t, e), e < n_in; output element s < n_out reads
 // column (base, stride) of where(s, row, base, stride), input sample d at
 // element base + d * stride, and goes to dst(t, s, value).  Triangles at or
-// past T stage zeros and are not written.  CHECKED: triangles holding an infinity
-// or NaN use every pair.
-template <int I, bool CHECKED, class Src, class Where, class Dst>
+// past T stage zeros and are not written.  Triangles holding an infinity or NaN
+// use every pair.
+template <int I, class Src, class Where, class Dst>
 __device__ __forceinline__ void map_triangles(const MapTables& m, int t0, int T, int n_in, int n_out, float* tile,
                                               Src src, Where where, Dst dst) {
     typedef typename MapVec<I>::type Vec;
@@ -225,28 +225,27 @@ __device__ __forceinline__ void map_triangles(const MapTables& m, int t0, int T,
 #pragma unroll
             for (int i = 0; i < I; ++i) {
                 q[i] = v[u][i];
-                if (CHECKED) odd = odd || !(fabsf(v[u][i]) <= 3.402823466e38f);
+                odd = odd || !(fabsf(v[u][i]) <= 3.402823466e38f);
             }
             *reinterpret_cast<Vec*>(tile + (size_t)(e0 + 32 * u) * I) = p;
         }
     }
     __syncwarp();
-    const MapRows r = CHECKED && __any_sync(0xffffffffu, odd) ? m.all : m.nonzero;
+    const MapRows r = __any_sync(0xffffffffu, odd) ? m.all : m.nonzero;
     for (int s = lane; s < n_out; s += 32) {
         int row, base, stride;
         float acc[I];
 #pragma unroll
         for (int i = 0; i < I; ++i) acc[i] = 0.f;
-        if (where(s, row, base, stride)) {
-            const int end = r.row[row + 1];
+        where(s, row, base, stride);
+        const int end = r.row[row + 1];
 #pragma unroll 2
-            for (int n = r.row[row]; n < end; ++n) {
-                const int2 e = r.ent[n];
-                const Vec x = *reinterpret_cast<const Vec*>(tile + (size_t)(base + e.x * stride) * I);
-                const float* xv = reinterpret_cast<const float*>(&x);
+        for (int n = r.row[row]; n < end; ++n) {
+            const int2 e = r.ent[n];
+            const Vec x = *reinterpret_cast<const Vec*>(tile + (size_t)(base + e.x * stride) * I);
+            const float* xv = reinterpret_cast<const float*>(&x);
 #pragma unroll
-                for (int i = 0; i < I; ++i) acc[i] = madd(acc[i], __int_as_float(e.y), xv[i]);
-            }
+            for (int i = 0; i < I; ++i) acc[i] = madd(acc[i], __int_as_float(e.y), xv[i]);
         }
 #pragma unroll
         for (int i = 0; i < I; ++i)

@@ -421,13 +421,12 @@ __global__ void __launch_bounds__(kMapWarps * 32) accumulate_map_kernel(int T, i
     float* tile = reinterpret_cast<float*>(map_smem + map_table_bytes(N, rows)) + (size_t)warp * n_in * I;
     const float inv_c = 1.f / (float)C;
     for (int64_t t = ((int64_t)blockIdx.x * kMapWarps + warp) * I; t < T; t += (int64_t)gridDim.x * kMapWarps * I)
-        map_triangles<I, true>(
+        map_triangles<I>(
             m, (int)t, T, n_in, n_out, tile, [&](int q, int e) { return __ldg(in + (size_t)q * n_in + e); },
             [&](int s, int& row, int& base, int& stride) {
                 row = (int)(((float)s + 0.5f) * inv_c);  // s / C (s + 1/2 keeps the product off the integers)
                 base = s - row * C;
                 stride = C;
-                return true;
             },
             [&](int q, int s, float v) {
                 float* o = out + (size_t)q * n_out + s;
