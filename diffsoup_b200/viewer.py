@@ -163,8 +163,8 @@ class Renderer:
         (as a tuple in that order)."""
         m = torch.as_tensor(mvps, dtype=torch.float32).reshape(-1, 4, 4)
         f = self._frame(m.shape[0], int(height), int(width))
-        # everything up to the one synchronisation is queued without waiting: the views' copy, the frame, the
-        # results' copies and the status word
+        # everything up to the one synchronisation is queued without waiting: the views' copy, the frame and the
+        # results' copies
         f.set_views(m, wait=False)
         f.status.zero_()
         f.run(want_rgb=rgb)
@@ -173,9 +173,7 @@ class Renderer:
             out.append(f.rgb.view(f.B, f.H, f.W, 3).clone())
         if gbuf:
             out.append(f.gbuf.view(f.B, f.H, f.W, 4).clone())
-        f.status_host.copy_(f.status, non_blocking=True)
-        torch.cuda.current_stream(self.device).synchronize()
-        if int(f.status_host) & _tiles.DS_STATUS_LIST_OVERFLOW:
+        if f.overflowed():  # reads the status word: the one synchronisation
             f.grow()  # this frame is exact all the same; the next ones bin without overflow
         return out[0] if len(out) == 1 else tuple(out)
 
@@ -211,7 +209,6 @@ class _Frame:
             self.rgb = torch.empty(self.num_pixels, 3, dtype=torch.float32, device=dev)
             self.rgba8 = torch.empty(self.num_pixels, 4, dtype=torch.uint8, device=dev)
             self.status = torch.zeros(1, dtype=torch.int32, device=dev)
-            self.status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)  # render()'s copy of it
         self.capacity = max(1 << 16, 8 * B * r.T)
         self._alloc()
 
