@@ -1099,7 +1099,10 @@ int ds_tiles_bin_report(int B, const ds_view_desc* views, int num_tiles, int V, 
     const int rc = ds_tiles_bin(B, views, num_tiles, V, pos, T, tri, workspace, workspace_bytes, list_capacity, status,
                                 stream);
     if (rc) return rc;
-    if (status_host != nullptr)
+    // not from a captured call: its replays would write to the word, whoever has it by then
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DS_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &capture));
+    if (status_host != nullptr && capture == cudaStreamCaptureStatusNone)
         DS_CUDA(cudaMemcpyAsync(status_host, status, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     return DS_OK;
 }

@@ -61,7 +61,7 @@ def view_table(hw: Sequence[Tuple[int, int]], device: torch.device):
 # slot is read without an event or a synchronisation.  A late copy into a slot
 # taken again shows the status of a call 256 earlier, so a capacity grows a call sooner
 # or later than it should; lists that do not fit are answered exactly all the same.
-# Captured calls take no slot: a replay would write to it whoever has it by then.
+# A captured call's slot stays at -1 (ds_tiles_bin_report leaves the copy out).
 _SLOTS = 256
 _slots: List = []  # [tensor, ctypes view], once allocated
 _slots_lock = threading.Lock()
@@ -141,15 +141,12 @@ def bin_views(pos: torch.Tensor, tri: torch.Tensor, hw: Sequence[Tuple[int, int]
     table, nt, npix, offs = view_table(hw, dev)
     cap = _capacity_for(dev, B, T)
     ws = _core.workspace(_core.lib.ds_tiles_workspace_size(B, T, nt, cap), dev)
-    word = None
-    if not torch.cuda.is_current_stream_capturing():
-        slots, slot = _status_slots(), next(_next_slot) % _SLOTS
-        slots[1][slot] = -1
-        word = slots[0].data_ptr() + 4 * slot
+    slots, slot = _status_slots(), next(_next_slot) % _SLOTS
+    slots[1][slot] = -1
     _core.check(_core.lib.ds_tiles_bin_report(B, _core.ptr(table), nt, V, _core.ptr(pos), T, _core.ptr(tri),
-                                              _core.ptr(ws), ws.numel(), cap, word, _core.stream()))
-    if word is not None:
-        _pending_status[_device_index(dev)] = (slot, cap)
+                                              _core.ptr(ws), ws.numel(), cap, slots[0].data_ptr() + 4 * slot,
+                                              _core.stream()))
+    _pending_status[_device_index(dev)] = (slot, cap)
     bins = Bins(B, T, V, hw, table, nt, npix, offs, cap, ws, pos, tri, key)
     _last = bins
     return bins

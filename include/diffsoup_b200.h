@@ -216,7 +216,8 @@ int ds_tiles_bin(int B, const ds_view_desc* views, int num_tiles, int V, const f
 
 /* ds_tiles_bin with the status word inside the workspace (cleared with the
  * bins, at ds_tiles_status_offset bytes) and an asynchronous copy of it to
- * *status_host (page-locked host memory that outlives the copy; NULL: none). */
+ * *status_host (page-locked host memory that outlives the copy; NULL, or
+ * while the stream is being captured: no copy). */
 size_t ds_tiles_status_offset(int B, int T, int num_tiles, int64_t list_capacity);
 int ds_tiles_bin_report(int B, const ds_view_desc* views, int num_tiles, int V, const float* pos, int T, const int* tri,
                         void* workspace, size_t workspace_bytes, int64_t list_capacity, int* status_host,

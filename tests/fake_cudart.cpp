@@ -114,6 +114,10 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStr
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)(handles += 16); return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t st) { line("record", st); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t, unsigned) { line("wait", st); return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) {
+    *s = cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t st) { line("synchronize", st); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t st) { line("memset", st); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t st) {
