@@ -756,7 +756,7 @@ def run_plain(sc, mlp, s, dev, n_views: int):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1)
     return {"value": n_views / (ms / 1000.0), "unit": "views/s", "views": n_views,
-            "path": "diffsoup_b200 drop-in API, one 800x800 view per call, FP32, eager autograd, torch ColorMLP"}
+            "path": "diffsoup_b200 drop-in API, one 800x800 view per call, FP32, eager autograd, ColorMLP on its FP32 kernels"}
 
 
 def run_render(dev, cpu_sample: bool = True, frames: int = 200):
