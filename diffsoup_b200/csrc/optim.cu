@@ -44,8 +44,12 @@ __device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, 
 // Parameters of one update, by value in the kernel's arguments.  Parameter i
 // takes blocks [first[i], first[i + 1]) of kAdamBlock elements.
 constexpr int kAdamMax = 32;
-constexpr int kAdamVecs = 2;  // float4 per thread
-constexpr int kAdamBlock = kThreads * 4 * kAdamVecs;
+constexpr int kAdamBlock = kThreads * 4;
+constexpr int kAdamPerSm = 5;  // resident CTAs (48 registers)
+// The grid is one wave of CTAs that stride over the blocks while what a step reads and writes stays in L2
+// (ten blocks a CTA: 7.6 M values, 121 MB); beyond that CTAs of four blocks, whose later ones fill the last
+// wave's gaps.  One parameter, us, a wave / fours: 5 M values 19 / 21, 7 M 35 / 38, 8 M 43.5 / 42, 20 M 103 / 93.
+constexpr unsigned kAdamWaveBlocks = 10, kAdamCtaBlocks = 4;
 
 struct AdamParams {
     float* p[kAdamMax];
@@ -58,58 +62,67 @@ struct AdamParams {
     int count;
 };
 
-// All parameters of a group in one launch.  Bound by memory: 28 bytes an element.
-// The bias corrections (two double-precision powers) are formed by one thread of
-// a block while the others' loads are in flight; formed by every thread they were most of the
-// time of a small parameter, and a launch per parameter the rest.  60,000
-// triangles of 24 samples x 8 channels with an MLP: 9 parameters 111 us of
-// kernels -> 66 us.
-__global__ void __launch_bounds__(kThreads) adam_kernel(const __grid_constant__ AdamParams a, double lr, double b1,
-                                                        double b2, float eps) {
+// All parameters of a group in one launch; a CTA strides over the blocks of kAdamBlock elements, one float4 a
+// thread.  Bound by memory: 28 bytes an element.  The bias corrections (two double-precision powers) are formed
+// by one thread of a CTA, once for each parameter that the CTA comes to, and before the loads, so that no
+// value is live across them: formed by every thread they were most of the time of a small parameter, by every
+// block (a grid of one block of 2,048 elements a CTA) 27 us for one parameter of 5 M values against 19 here, with the
+// loads in flight (spilled at 48 registers) 21.  Unaligned, or a parameter's last block: the same loads four
+// bytes wide, all of a thread's in flight (5 M values 39 us in a loop -> 21).
+__global__ void __launch_bounds__(kThreads, kAdamPerSm)
+    adam_kernel(const __grid_constant__ AdamParams a, double lr, double b1, double b2, float eps) {
     __shared__ AdamScale s_scale;
-    int q = 0;
-    while (blockIdx.x >= a.first[q + 1]) ++q;  // block-uniform
-    const int64_t base = (int64_t)(blockIdx.x - a.first[q]) * kAdamBlock, n = a.n[q];
-    float* __restrict__ p = a.p[q];
-    const float* __restrict__ g = a.g[q];
-    float* __restrict__ m = a.m[q];
-    float* __restrict__ v = a.v[q];
-    const bool vec = (((uintptr_t)p | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v) & 15) == 0;
-    if (vec && base + kAdamBlock <= n) {
-        float4 pp[kAdamVecs], gg[kAdamVecs], mm[kAdamVecs], vv[kAdamVecs];
-        const int64_t o = base / 4 + threadIdx.x;
-#pragma unroll
-        for (int u = 0; u < kAdamVecs; ++u) {
-            pp[u] = reinterpret_cast<const float4*>(p)[o + u * kThreads];
-            gg[u] = reinterpret_cast<const float4*>(g)[o + u * kThreads];
-            mm[u] = reinterpret_cast<const float4*>(m)[o + u * kThreads];
-            vv[u] = reinterpret_cast<const float4*>(v)[o + u * kThreads];
+    int q = 0, scaled = -1;
+    AdamScale s;
+    for (unsigned blk = blockIdx.x; blk < a.first[a.count]; blk += gridDim.x) {
+        while (blk >= a.first[q + 1]) ++q;  // CTA-uniform
+        if (scaled != q) {
+            __syncthreads();  // every thread has taken the last parameter's
+            if (threadIdx.x == 0) s_scale = adam_scale(a.step[q], lr, b1, b2);
+            __syncthreads();
+            s = s_scale;
+            scaled = q;
         }
-        if (threadIdx.x == 0) s_scale = adam_scale(a.step[q], lr, b1, b2);
-        __syncthreads();
-        const AdamScale s = s_scale;
+        const int64_t base = (int64_t)(blk - a.first[q]) * kAdamBlock, left = a.n[q] - base;
+        float* __restrict__ p = a.p[q] + base;
+        const float* __restrict__ g = a.g[q] + base;
+        float* __restrict__ m = a.m[q] + base;
+        float* __restrict__ v = a.v[q] + base;
+        const bool full = left >= kAdamBlock && (((uintptr_t)p | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v) & 15) == 0;
+        const int count = left < kAdamBlock ? (int)left : kAdamBlock;
+        float pp[4], gg[4], mm[4], vv[4];
+        if (full) {
+            *reinterpret_cast<float4*>(pp) = reinterpret_cast<const float4*>(p)[threadIdx.x];
+            *reinterpret_cast<float4*>(gg) = reinterpret_cast<const float4*>(g)[threadIdx.x];
+            *reinterpret_cast<float4*>(mm) = reinterpret_cast<const float4*>(m)[threadIdx.x];
+            *reinterpret_cast<float4*>(vv) = reinterpret_cast<const float4*>(v)[threadIdx.x];
+        } else {  // a parameter's last block, or an unaligned one
 #pragma unroll
-        for (int u = 0; u < kAdamVecs; ++u) {
-            adam_one(pp[u].x, gg[u].x, mm[u].x, vv[u].x, s, eps);
-            adam_one(pp[u].y, gg[u].y, mm[u].y, vv[u].y, s, eps);
-            adam_one(pp[u].z, gg[u].z, mm[u].z, vv[u].z, s, eps);
-            adam_one(pp[u].w, gg[u].w, mm[u].w, vv[u].w, s, eps);
-            reinterpret_cast<float4*>(p)[o + u * kThreads] = pp[u];
-            reinterpret_cast<float4*>(m)[o + u * kThreads] = mm[u];
-            reinterpret_cast<float4*>(v)[o + u * kThreads] = vv[u];
+            for (int k = 0; k < 4; ++k) {
+                const int i = threadIdx.x + k * kThreads;
+                pp[k] = i < count ? p[i] : 0.0f;
+                gg[k] = i < count ? g[i] : 0.0f;
+                mm[k] = i < count ? m[i] : 0.0f;
+                vv[k] = i < count ? v[i] : 0.0f;
+            }
         }
-        return;
-    }
-    if (threadIdx.x == 0) s_scale = adam_scale(a.step[q], lr, b1, b2);
-    __syncthreads();
-    const AdamScale s = s_scale;
-    const int64_t end = base + kAdamBlock < n ? base + kAdamBlock : n;
-    for (int64_t i = base + threadIdx.x; i < end; i += kThreads) {
-        float pp = p[i], mm = m[i], vv = v[i];
-        adam_one(pp, g[i], mm, vv, s, eps);
-        p[i] = pp;
-        m[i] = mm;
-        v[i] = vv;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) adam_one(pp[k], gg[k], mm[k], vv[k], s, eps);
+        if (full) {
+            reinterpret_cast<float4*>(p)[threadIdx.x] = *reinterpret_cast<float4*>(pp);
+            reinterpret_cast<float4*>(m)[threadIdx.x] = *reinterpret_cast<float4*>(mm);
+            reinterpret_cast<float4*>(v)[threadIdx.x] = *reinterpret_cast<float4*>(vv);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int i = threadIdx.x + k * kThreads;
+                if (i < count) {
+                    p[i] = pp[k];
+                    m[i] = mm[k];
+                    v[i] = vv[k];
+                }
+            }
+        }
     }
 }
 
@@ -202,8 +215,11 @@ int ds_adam_step_multi(int count, float* const* params_host, const float* const*
             a.first[k + 1] = a.first[k] + (unsigned)blocks;
             ++i;
         }
-        if (a.first[a.count] > 0)
-            adam_kernel<<<a.first[a.count], kThreads, 0, st>>>(a, lr, beta1, beta2, (float)eps);
+        const unsigned all = a.first[a.count], wave = (unsigned)sm_count() * kAdamPerSm;
+        const unsigned grid = all <= wave                    ? all
+                              : all / kAdamWaveBlocks < wave ? wave
+                                                             : (all + kAdamCtaBlocks - 1) / kAdamCtaBlocks;
+        if (all > 0) adam_kernel<<<grid, kThreads, 0, st>>>(a, lr, beta1, beta2, (float)eps);
         advance_steps_kernel<<<1, 32, 0, st>>>(a);
     }
     return check_launch("adam_step");
