@@ -287,9 +287,14 @@ __global__ void __launch_bounds__(kThreads) color_backward_kernel(int64_t n, con
 // atomics, which bound the kernel above: a warp takes 8x4 pixels of a view,
 // groups those of one (triangle, cell), and an item (group, sample and, of four or more
 // channels, a group of four) sums its members' weighted rows and issues the atomics of
-// one row.  Where less than a third of the warp's pixels would be merged they go out
-// per pixel.  4 views of 800x800, 7 channels: 103 -> 43 us.
+// one row, its members shared by up to eight lanes where there are few items (801x603, one cell a
+// triangle of 64 pixels, 7 / 4 channels: 20.9 / 18.8 us, 12.7 / 12.7 so).  Where less than a third of the warp's pixels
+// would be merged they go out per pixel.  4 views of 800x800, 7 channels: 103 -> 43 us.
 constexpr int kMergeRow = 32;  // channels up to which the rows are staged
+// Quads of channels from which unmerged pixels go out as items too, the lanes of a row beside one another: triangle IDs
+// drawn by pixel, two views of 800x800, 60,000 / 100 triangles: 32 channels 242 / 416 us a lane per pixel, 201 / 191 as
+// items; 16: 97 / 215, 95 / 96; 12: 74 / 165, 76 / 95 (one 801x603 view of 5,000: 35, 37); 8: 49 / 171, 57 / 83.
+constexpr int kMergeQuads = 4;
 
 // Floats between the staged rows: the row and its three weights, an odd number of floats, or of
 // groups of four, so that the rows of eight lanes fall in different banks (12 channels 88 us with 16 floats,
@@ -353,8 +358,14 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
         leader = covered && lane == __ffs(peers) - 1;
         leaders = __ballot_sync(0xffffffffu, leader);
     }
-    const int groups = __popc(leaders);
-    if (3 * groups > 2 * __popc(live)) {
+    const int Q = ROW7 ? 1 : C / 4;
+    int groups = __popc(leaders);
+    if (3 * groups > 2 * __popc(live) && Q >= kMergeQuads) {
+        peers = 1u << lane;  // each pixel an item's only member
+        leader = covered;
+        leaders = live;
+        groups = __popc(live);
+    } else if (3 * groups > 2 * __popc(live)) {
         if (!covered) return;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -376,21 +387,25 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
         g[0] = (int)peers; g[1] = t; g[2] = (int)idx[0]; g[3] = (int)idx[1]; g[4] = (int)idx[2];
     }
     __syncwarp();
-    const int Q = ROW7 ? 1 : C / 4;
-    for (int n = lane; n < groups * 3 * Q; n += 32) {
-        const int gi = n / (3 * Q), rest = n - gi * 3 * Q, k = rest / Q, c = (rest - k * Q) * 4;
+    const int items = groups * 3 * Q, parts = items > 16 ? 1 : items > 8 ? 2 : items > 4 ? 4 : 8;
+    const unsigned part = (0xffffffffu / ((1u << parts) - 1u)) << (lane & (parts - 1));
+    for (int n0 = 0; n0 < items; n0 += 32 / parts) {  // warp-uniform
+        const int n = n0 + lane / parts, gi = n / (3 * Q), rest = n - gi * 3 * Q, k = rest / Q, c = (rest - k * Q) * 4;
         const int* g = meta + gi * 5;
-        unsigned members = (unsigned)g[0];
-        const size_t at = (size_t)g[1] * S + (size_t)g[2 + k];
         float v[ROW7 ? 7 : 4];
 #pragma unroll
         for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] = 0.f;
-        for (; members != 0; members &= members - 1u) {
+        for (unsigned members = n < items ? (unsigned)g[0] & part : 0u; members != 0; members &= members - 1u) {
             const float* m = rows + (__ffs(members) - 1) * stride;
             const float wk = m[C + k];
 #pragma unroll
             for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] = fmaf(wk, m[c + j], v[j]);
         }
+        for (int d = 1; d < parts; d += d)
+#pragma unroll
+            for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], d);
+        if (n >= items || (lane & (parts - 1)) != 0) continue;
+        const size_t at = (size_t)g[1] * S + (size_t)g[2 + k];
         if (ROW7) Row7((uint32_t)at).add(grad_feat + at * 7, v, 1.f);
         else atomicAdd(reinterpret_cast<float4*>(grad_feat + at * C + c), make_float4(v[0], v[1], v[2], v[3]));
     }
