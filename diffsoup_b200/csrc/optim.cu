@@ -12,7 +12,6 @@
 
 namespace dsb {
 
-// Bias corrections of step t (the count after this update's increment).
 struct AdamScale {
     float b1, b2, one_m_b1, one_m_b2, step_size, bc2_sqrt;
 };
@@ -20,17 +19,19 @@ struct AdamScale {
 // The hyperparameters arrive in double, as torch's Python scalars: the
 // complements 1 - beta are formed in double and then rounded, like torch's
 // alpha / weight arguments.
-__device__ __forceinline__ AdamScale adam_scale(const int* step, double lr, double b1, double b2) {
-    const double t = (double)(*step + 1);
-    const double bc1 = 1.0 - pow(b1, t), bc2 = 1.0 - pow(b2, t);
+__device__ __forceinline__ AdamScale adam_betas(double b1, double b2) {
     AdamScale s;
     s.b1 = (float)b1;
     s.b2 = (float)b2;
     s.one_m_b1 = (float)(1.0 - b1);
     s.one_m_b2 = (float)(1.0 - b2);
-    s.step_size = (float)(lr / bc1);
-    s.bc2_sqrt = (float)sqrt(bc2);
     return s;
+}
+
+// A bias correction of step t (the count after this update's increment): lr / (1 - b1^t), or sqrt(1 - b2^t).
+__device__ __forceinline__ float adam_correction(const int* step, double lr, double b, bool second) {
+    const double bc = 1.0 - pow(b, (double)(*step + 1));
+    return (float)(second ? sqrt(bc) : lr / bc);
 }
 
 // torch.optim.Adam, one element: m <- m + (1-b1)(g - m), v <- b2 v + (1-b2) g^2,
@@ -48,7 +49,7 @@ constexpr int kAdamBlock = kThreads * 4;
 constexpr int kAdamPerSm = 5;  // resident CTAs (48 registers)
 // The grid is one wave of CTAs that stride over the blocks while what a step reads and writes stays in L2
 // (ten blocks a CTA: 7.6 M values, 121 MB); beyond that CTAs of four blocks, whose later ones fill the last
-// wave's gaps.  One parameter, us, a wave / fours: 5 M values 19 / 21, 7 M 35 / 38, 8 M 43.5 / 42, 20 M 103 / 93.
+// wave's gaps.  One parameter, us, a wave / fours: 5 M values 19 / 21, 7 M 34 / 38, 8 M 43 / 41, 20 M 103 / 91.
 constexpr unsigned kAdamWaveBlocks = 10, kAdamCtaBlocks = 4;
 
 struct AdamParams {
@@ -64,23 +65,27 @@ struct AdamParams {
 
 // All parameters of a group in one launch; a CTA strides over the blocks of kAdamBlock elements, one float4 a
 // thread.  Bound by memory: 28 bytes an element.  The bias corrections (two double-precision powers) are formed
-// by one thread of a CTA, once for each parameter that the CTA comes to, and before the loads, so that no
+// by two warps of a CTA, once for each parameter that the CTA comes to, and before the loads, so that no
 // value is live across them: formed by every thread they were most of the time of a small parameter, by every
 // block (a grid of one block of 2,048 elements a CTA) 27 us for one parameter of 5 M values against 19 here, with the
 // loads in flight (spilled at 48 registers) 21.  Unaligned, or a parameter's last block: the same loads four
 // bytes wide, all of a thread's in flight (5 M values 39 us in a loop -> 21).
 __global__ void __launch_bounds__(kThreads, kAdamPerSm)
     adam_kernel(const __grid_constant__ AdamParams a, double lr, double b1, double b2, float eps) {
-    __shared__ AdamScale s_scale;
+    __shared__ float s_scale[2];
     int q = 0, scaled = -1;
-    AdamScale s;
+    AdamScale s = adam_betas(b1, b2);
     for (unsigned blk = blockIdx.x; blk < a.first[a.count]; blk += gridDim.x) {
         while (blk >= a.first[q + 1]) ++q;  // CTA-uniform
         if (scaled != q) {
             __syncthreads();  // every thread has taken the last parameter's
-            if (threadIdx.x == 0) s_scale = adam_scale(a.step[q], lr, b1, b2);
+            if (threadIdx.x == 0 || threadIdx.x == 32) {
+                const int k = threadIdx.x >> 5;
+                s_scale[k] = adam_correction(a.step[q], lr, k ? b2 : b1, k);
+            }
             __syncthreads();
-            s = s_scale;
+            s.step_size = s_scale[0];
+            s.bc2_sqrt = s_scale[1];
             scaled = q;
         }
         const int64_t base = (int64_t)(blk - a.first[q]) * kAdamBlock, left = a.n[q] - base;
