@@ -139,6 +139,8 @@ __device__ __forceinline__ void zero_rows(float* g, uint32_t C, unsigned rows) {
 
 // color_kernel with every pixel written (background pixels zero): no zeroed
 // buffer and no read of it.  The covered pixels' rows are stored
+//   kLookupNarrow  by their lanes, four channels at a time, background rows by the same stores: rows of four
+//                channels are half a sector, and apart from one another the two kinds of rows write it twice;
 //   kLookupVec4  by their lanes, four channels at a time;
 //   kLookupRow7  (seven channels of an aligned table, read as Row7) and
 //   kLookupTile  through shared memory, so that a warp's 32 rows leave as one run of
@@ -150,10 +152,13 @@ __device__ __forceinline__ void zero_rows(float* g, uint32_t C, unsigned rows) {
 // 32 channels: 43 us with a zeroed buffer, 91 with every lane zeroing its own row, 32 so; 60,000
 // triangles on nine tenths: 181, 115 and 105.  4 views of 800x800, 7 channels: 53, 12 of them
 // zeroing, -> 39 us.
-enum { kLookupVec4, kLookupRow7, kLookupTile, kLookupRows };
+enum { kLookupNarrow, kLookupVec4, kLookupRow7, kLookupTile, kLookupRows };
 // Channels up to which kLookupTile is taken: its shared memory stays below the 48 KB of a plain launch.  31
 // channels on nine tenths as above: 267 us with a zeroed buffer, 309 by lanes, 152 through the tile.
 constexpr int kColorTile = 32;
+// Channels up to which kLookupNarrow is taken.  4 views of 800x800, 15,000 triangles on half of the pixels, 4 / 8
+// channels: 18 / 33 us, 25 / 37 as kLookupVec4; 894x670, 5 views, 16: 68, 62.
+constexpr int kLookupNarrowest = 8;
 
 template <int MODE>
 __global__ void __launch_bounds__(kThreads) color_set_kernel(int64_t n, const float* __restrict__ rast, uint32_t lo,
@@ -165,8 +170,30 @@ __global__ void __launch_bounds__(kThreads) color_set_kernel(int64_t n, const fl
     const int lane = threadIdx.x & 31;
     const int64_t p0 = p - lane;
     const bool in = p < n;
+    if (MODE == kLookupNarrow && !in) return;
     const float4 r = in ? reinterpret_cast<const float4*>(rast)[p] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int t = (int)r.w - 1;
+    if (MODE == kLookupNarrow) {
+        uint32_t idx[3]; float w[3];
+        lattice_cell(r.x, r.y, lo, idx, w);
+        for (int c = 0; c < C; c += 4) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint32_t off = 0;
+            for (uint32_t l = lo; t >= 0 && l <= hi; ++l) {
+                if (lo < hi) lattice_cell(r.x, r.y, l, idx, w);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float4 f =
+                        __ldg(reinterpret_cast<const float4*>(feat + ((size_t)t * S + off + idx[k]) * C + c));
+                    acc.x = madd(acc.x, w[k], f.x); acc.y = madd(acc.y, w[k], f.y);
+                    acc.z = madd(acc.z, w[k], f.z); acc.w = madd(acc.w, w[k], f.w);
+                }
+                off += feats_at_level(l);
+            }
+            *reinterpret_cast<float4*>(out + (size_t)p * C + c) = acc;
+        }
+        return;
+    }
     const unsigned zero = __ballot_sync(0xffffffffu, in && (t < 0 || MODE == kLookupRows));
     if (STAGED ? zero == 0xffffffffu : zero != 0u) zero_rows(out + (size_t)p0 * C, (uint32_t)C, zero);
     if (MODE == kLookupRows) __syncwarp();
@@ -645,10 +672,12 @@ int ds_multires_triangle_color_set(int B, int H, int W, const float* rast, int m
     DS_CHECK_ARG(aligned16(rast), "multires_triangle_color: rast not 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
     const size_t tile = (size_t)kThreads * C * sizeof(float);
-    const auto kernel = C % 4 == 0 && aligned16(features) && aligned16(out) ? color_set_kernel<kLookupVec4>
-                        : C == 7 && aligned16(features)                     ? color_set_kernel<kLookupRow7>
-                        : C <= kColorTile                                   ? color_set_kernel<kLookupTile>
-                                                                            : color_set_kernel<kLookupRows>;
+    const bool vec = C % 4 == 0 && aligned16(features) && aligned16(out);
+    const auto kernel = vec && C <= kLookupNarrowest    ? color_set_kernel<kLookupNarrow>
+                        : vec                           ? color_set_kernel<kLookupVec4>
+                        : C == 7 && aligned16(features) ? color_set_kernel<kLookupRow7>
+                        : C <= kColorTile               ? color_set_kernel<kLookupTile>
+                                                        : color_set_kernel<kLookupRows>;
     const bool staged = kernel == color_set_kernel<kLookupRow7> || kernel == color_set_kernel<kLookupTile>;
     kernel<<<blocks_for(n), kThreads, staged ? tile : 0, st>>>(n, rast, min_level, max_level, S, C, features, out);
     return check_launch("multires_triangle_color");
