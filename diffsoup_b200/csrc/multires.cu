@@ -314,19 +314,54 @@ __global__ void __launch_bounds__(kThreads) color_backward_kernel(int64_t n, con
 // atomics, which bound the kernel above: a warp takes 8x4 pixels of a view,
 // groups those of one (triangle, cell), and an item (group, sample and, of four or more
 // channels, a group of four) sums its members' weighted rows and issues the atomics of
-// one row, its members shared by up to eight lanes where there are few items (801x603, one cell a
-// triangle of 64 pixels, 7 / 4 channels: 20.9 / 18.8 us, 12.7 / 12.7 so).  Where less than a third of the warp's pixels
+// one row, its members shared by eight or four lanes where there are up to four or eight items (801x603, one cell a
+// triangle of 64 pixels, 7 / 4 channels: 20.9 / 18.8 us, 12.7 / 12.7 so; sharing by a run-time count at
+// more items cost 10% where cells are small).  Where less than a third of the warp's pixels
 // would be merged they go out per pixel.  4 views of 800x800, 7 channels: 103 -> 43 us.
 constexpr int kMergeRow = 32;  // channels up to which the rows are staged
 // Quads of channels from which unmerged pixels go out as items too, the lanes of a row beside one another: triangle IDs
-// drawn by pixel, two views of 800x800, 60,000 / 100 triangles: 32 channels 242 / 416 us a lane per pixel, 201 / 191 as
-// items; 16: 97 / 215, 95 / 96; 12: 74 / 165, 76 / 95 (one 801x603 view of 5,000: 35, 37); 8: 49 / 171, 57 / 83.
-constexpr int kMergeQuads = 4;
+// drawn by pixel, two views of 800x800, 60,000 / 100 triangles, 32 channels: 237 / 414 us a lane per pixel, 207 / 191 as
+// items.  Narrower rows are the faster by pixel where a scene's triangles leave few warps unmerged (894x670, 12,000
+// triangles, 16 channels at level 3: 60 us, 72 as items).
+constexpr int kMergeQuads = 8;
 
 // Floats between the staged rows: the row and its three weights, an odd number of floats, or of
 // groups of four, so that the rows of eight lanes fall in different banks (12 channels 88 us with 16 floats,
 // 72 with 20).
 __host__ __device__ constexpr int merge_stride(int C) { return C == 7 ? 11 : C + 4 + (C & 4); }
+
+// The items (group, sample, quad) of a warp, each by 1 << SHARE lanes.
+template <bool ROW7, int SHARE>
+__device__ __forceinline__ void merge_items(int items, int Q, int lane, int stride, const float* rows, const int* meta,
+                                            uint32_t S, int C, float* __restrict__ grad_feat) {
+    constexpr unsigned kPart =
+        SHARE == 0 ? 0xffffffffu : SHARE == 1 ? 0x55555555u : SHARE == 2 ? 0x11111111u : 0x01010101u;
+    const int first = lane >> SHARE, own = lane & ((1 << SHARE) - 1);
+    for (int n0 = 0; n0 < items; n0 += 32 >> SHARE) {  // warp-uniform
+        const int n = n0 + first;
+        const bool some = n < items;
+        if (SHARE == 0 && !some) break;
+        const int gi = n / (3 * Q), rest = n - gi * 3 * Q, k = rest / Q, c = (rest - k * Q) * 4;
+        const int* g = meta + gi * 5;
+        float v[ROW7 ? 7 : 4];
+#pragma unroll
+        for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] = 0.f;
+        for (unsigned members = some ? (unsigned)g[0] & (kPart << own) : 0u; members != 0; members &= members - 1u) {
+            const float* m = rows + (__ffs(members) - 1) * stride;
+            const float wk = m[C + k];
+#pragma unroll
+            for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] = fmaf(wk, m[c + j], v[j]);
+        }
+#pragma unroll
+        for (int d = 1; d < 1 << SHARE; d += d)
+#pragma unroll
+            for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], d);
+        if (!some || own != 0) continue;
+        const size_t at = (size_t)g[1] * S + (size_t)g[2 + k];
+        if (ROW7) Row7((uint32_t)at).add(grad_feat + at * 7, v, 1.f);
+        else atomicAdd(reinterpret_cast<float4*>(grad_feat + at * C + c), make_float4(v[0], v[1], v[2], v[3]));
+    }
+}
 
 template <bool ROW7>
 __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, int W, int bx, int64_t blocks, int per_view,
@@ -372,15 +407,19 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
         covered ? ((unsigned long long)(unsigned)t << 34) | ((unsigned long long)(idx[0] & 0xffffu) << 18) |
                       ((unsigned long long)(idx[1] & 0xffffu) << 2) | (idx[2] == idx[0] ? 2u : (idx[2] > idx[1] ? 1u : 0u))
                 : ~0ull;
-    // where few pixels share a cell with the pixel beside or above them, the grouping is not tried: it is slow
-    // for many different keys (60,000 triangles, one a pixel, two views of 800x800, 4 channels: 34 us without
-    // grouping, 41 with it, 29 so; 8 channels 47, 54, 47)
-    const unsigned long long beside = __shfl_down_sync(0xffffffffu, key, 1), above = __shfl_down_sync(0xffffffffu, key, 8);
-    const int pairs = __popc(__ballot_sync(0xffffffffu, covered && (lane & 7) != 7 && beside == key)) +
-                      __popc(__ballot_sync(0xffffffffu, covered && lane < 24 && above == key));
+    // Grouping is tried where it can merge a third of the pixels: as many must share a cell with the pixel beside or
+    // above them (by a hash of the key), for a cell's pixels hang together.  One quad a row, whose atomics are
+    // cheapest, asks for as many such pairs as pixels.  It is slow for many different keys (60,000 triangles, one a pixel,
+    // two views of 800x800, 4 channels: 34 us without grouping, 41 with it always, 29 so).  4 channels of 4 views of
+    // 800x800 of a shell of 15,000 triangles / a box of 60,000, pairs for a third of the pixels 40 / 62 us, for all 33 / 52,
+    // never grouped 35 / 68, a thread per pixel without staging 29 / 64.
+    const unsigned mix = (unsigned)key ^ ((unsigned)(key >> 32) * 0x9e3779b1u);
+    const unsigned beside = __shfl_down_sync(0xffffffffu, mix, 1), above = __shfl_down_sync(0xffffffffu, mix, 8);
+    const int pairs = __popc(__ballot_sync(0xffffffffu, covered && (lane & 7) != 7 && beside == mix)) +
+                      __popc(__ballot_sync(0xffffffffu, covered && lane < 24 && above == mix));
     unsigned peers = 0u, leaders = live;
     bool leader = false;
-    if (6 * pairs >= __popc(live)) {
+    if ((C == 4 ? 1 : 3) * pairs >= __popc(live)) {
         peers = __match_any_sync(0xffffffffu, key);
         leader = covered && lane == __ffs(peers) - 1;
         leaders = __ballot_sync(0xffffffffu, leader);
@@ -414,28 +453,15 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
         g[0] = (int)peers; g[1] = t; g[2] = (int)idx[0]; g[3] = (int)idx[1]; g[4] = (int)idx[2];
     }
     __syncwarp();
-    const int items = groups * 3 * Q, parts = items > 16 ? 1 : items > 8 ? 2 : items > 4 ? 4 : 8;
-    const unsigned part = (0xffffffffu / ((1u << parts) - 1u)) << (lane & (parts - 1));
-    for (int n0 = 0; n0 < items; n0 += 32 / parts) {  // warp-uniform
-        const int n = n0 + lane / parts, gi = n / (3 * Q), rest = n - gi * 3 * Q, k = rest / Q, c = (rest - k * Q) * 4;
-        const int* g = meta + gi * 5;
-        float v[ROW7 ? 7 : 4];
-#pragma unroll
-        for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] = 0.f;
-        for (unsigned members = n < items ? (unsigned)g[0] & part : 0u; members != 0; members &= members - 1u) {
-            const float* m = rows + (__ffs(members) - 1) * stride;
-            const float wk = m[C + k];
-#pragma unroll
-            for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] = fmaf(wk, m[c + j], v[j]);
-        }
-        for (int d = 1; d < parts; d += d)
-#pragma unroll
-            for (int j = 0; j < (ROW7 ? 7 : 4); ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], d);
-        if (n >= items || (lane & (parts - 1)) != 0) continue;
-        const size_t at = (size_t)g[1] * S + (size_t)g[2 + k];
-        if (ROW7) Row7((uint32_t)at).add(grad_feat + at * 7, v, 1.f);
-        else atomicAdd(reinterpret_cast<float4*>(grad_feat + at * C + c), make_float4(v[0], v[1], v[2], v[3]));
-    }
+    const int items = groups * 3 * Q;
+    if (items <= 4)
+        merge_items<ROW7, 3>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
+    else if (items <= 8)
+        merge_items<ROW7, 2>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
+    else if (Q == 1 && items <= 16 && !ROW7)  // small cells: 52 us for 56 (the box above), 21 for 23 (a view of 801x603)
+        merge_items<ROW7, 1>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
+    else
+        merge_items<ROW7, 0>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
 }
 
 // The level accumulation through the map's tables (lattice_map.cuh), forward
