@@ -312,13 +312,17 @@ __global__ void __launch_bounds__(kThreads) color_backward_kernel(int64_t n, con
 
 // The scatter at one level with the pixels of a lattice cell summed before the
 // atomics, which bound the kernel above: a warp takes 8x4 pixels of a view,
-// groups those of one (triangle, cell), and an item (group, sample and, of four or more
+// groups those of one (triangle, cell), and an item (group, sample and, of eight or more
 // channels, a group of four) sums its members' weighted rows and issues the atomics of
 // one row, its members shared by eight or four lanes where there are up to four or eight items (801x603, one cell a
-// triangle of 64 pixels, 7 / 4 channels: 20.9 / 18.8 us, 12.7 / 12.7 so; sharing by a run-time count at
-// more items cost 10% where cells are small).  Where less than a third of the warp's pixels
-// would be merged they go out per pixel.  4 views of 800x800, 7 channels: 103 -> 43 us.
+// triangle of 64 pixels, 7 channels: 21 us, 13 so; sharing by a run-time count at more items cost 10%
+// where cells are small).  Where less than a third of the warp's pixels would be merged they go out
+// per pixel.  4 views of 800x800, 7 channels: 103 -> 43 us.
 constexpr int kMergeRow = 32;  // channels up to which the rows are staged
+// Rows of at least this many channels are merged: one vector atomic a sample is as cheap as the merging. 4 channels, a
+// thread per pixel / merged: shell of 15,000 triangles, 4 views of 800x800, 29 / 33 us, of 3,000, one view of 801x603 at
+// level 1, 15 / 21, boxes of 60,000 and 50,000 64 / 52, 117 / 93; 8 channels, the first, 60 / 49.
+constexpr int kMergeFrom = 7;
 // Quads of channels from which unmerged pixels go out as items too, the lanes of a row beside one another: triangle IDs
 // drawn by pixel, two views of 800x800, 60,000 / 100 triangles, 32 channels: 237 / 414 us a lane per pixel, 207 / 191 as
 // items.  Narrower rows are the faster by pixel where a scene's triangles leave few warps unmerged (894x670, 12,000
@@ -334,8 +338,7 @@ __host__ __device__ constexpr int merge_stride(int C) { return C == 7 ? 11 : C +
 template <bool ROW7, int SHARE>
 __device__ __forceinline__ void merge_items(int items, int Q, int lane, int stride, const float* rows, const int* meta,
                                             uint32_t S, int C, float* __restrict__ grad_feat) {
-    constexpr unsigned kPart =
-        SHARE == 0 ? 0xffffffffu : SHARE == 1 ? 0x55555555u : SHARE == 2 ? 0x11111111u : 0x01010101u;
+    constexpr unsigned kPart = SHARE == 0 ? 0xffffffffu : SHARE == 2 ? 0x11111111u : 0x01010101u;
     const int first = lane >> SHARE, own = lane & ((1 << SHARE) - 1);
     for (int n0 = 0; n0 < items; n0 += 32 >> SHARE) {  // warp-uniform
         const int n = n0 + first;
@@ -408,18 +411,15 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
                       ((unsigned long long)(idx[1] & 0xffffu) << 2) | (idx[2] == idx[0] ? 2u : (idx[2] > idx[1] ? 1u : 0u))
                 : ~0ull;
     // Grouping is tried where it can merge a third of the pixels: as many must share a cell with the pixel beside or
-    // above them (by a hash of the key), for a cell's pixels hang together.  One quad a row, whose atomics are
-    // cheapest, asks for as many such pairs as pixels.  It is slow for many different keys (60,000 triangles, one a pixel,
-    // two views of 800x800, 4 channels: 34 us without grouping, 41 with it always, 29 so).  4 channels of 4 views of
-    // 800x800 of a shell of 15,000 triangles / a box of 60,000, pairs for a third of the pixels 40 / 62 us, for all 33 / 52,
-    // never grouped 35 / 68, a thread per pixel without staging 29 / 64.
+    // above them (by a hash of the key), for a cell's pixels hang together.  It is slow for many different keys
+    // (60,000 triangles, one a pixel, two views of 800x800, 8 channels: 47 us without it, 54 with it always, 49 so).
     const unsigned mix = (unsigned)key ^ ((unsigned)(key >> 32) * 0x9e3779b1u);
     const unsigned beside = __shfl_down_sync(0xffffffffu, mix, 1), above = __shfl_down_sync(0xffffffffu, mix, 8);
     const int pairs = __popc(__ballot_sync(0xffffffffu, covered && (lane & 7) != 7 && beside == mix)) +
                       __popc(__ballot_sync(0xffffffffu, covered && lane < 24 && above == mix));
     unsigned peers = 0u, leaders = live;
     bool leader = false;
-    if ((C == 4 ? 1 : 3) * pairs >= __popc(live)) {
+    if (3 * pairs >= __popc(live)) {
         peers = __match_any_sync(0xffffffffu, key);
         leader = covered && lane == __ffs(peers) - 1;
         leaders = __ballot_sync(0xffffffffu, leader);
@@ -458,8 +458,6 @@ __global__ void __launch_bounds__(kThreads) color_backward_merge_kernel(int H, i
         merge_items<ROW7, 3>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
     else if (items <= 8)
         merge_items<ROW7, 2>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
-    else if (Q == 1 && items <= 16 && !ROW7)  // small cells: 52 us for 56 (the box above), 21 for 23 (a view of 801x603)
-        merge_items<ROW7, 1>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
     else
         merge_items<ROW7, 0>(items, Q, lane, stride, rows, meta, S, C, grad_feat);
 }
@@ -723,8 +721,8 @@ int ds_backward_multires_triangle_color(int B, int H, int W, const float* rast, 
     // ID buffer's floats count to 2^24), and channels that fit its rows
     const int bx = (W + 7) / 8, by = (H + 3) / 4;
     const int64_t nb = (int64_t)B * bx * by;
-    if (min_level == max_level && max_level <= 8 && C <= kMergeRow && (vec || (C == 7 && aligned16(grad_features))) &&
-        (int64_t)bx * by <= 0x7fffffff && nb <= 0x7fffffff) {
+    if (min_level == max_level && max_level <= 8 && C >= kMergeFrom && C <= kMergeRow &&
+        (vec || (C == 7 && aligned16(grad_features))) && (int64_t)bx * by <= 0x7fffffff && nb <= 0x7fffffff) {
         const size_t smem = (size_t)(kThreads / 32) * (32 * merge_stride(C) + 160) * sizeof(float);
         const unsigned grid = (unsigned)((nb + kThreads / 32 - 1) / (kThreads / 32));
         if (C == 7)
